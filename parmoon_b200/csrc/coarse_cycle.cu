@@ -525,28 +525,35 @@ static int cluster_ctas() {
 }
 
 // the highest level that, with every level below it, fits the cluster launch
-// (0: none -- the level-by-level path runs).  PMG_COARSE_CLUSTER=<ctas>[:<max
-// rows>] chooses the shape: the default "8:8192" runs the levels of at most
-// 8192 rows on an 8-CTA cluster (measured: 64^3 Q2 FP32 V-cycle 4.17 ms
-// against 4.31 ms level by level; larger levels stream more matrix per colour
-// pass than one GPC's share of L2 bandwidth carries faster than the 148-SM
-// colour launches); "1" runs the levels of at most CC_ONE_CTA_ROWS rows on one
-// CTA, "16" (2, 4, 8) every level whose iterates fit CC_SMEM_X on a cluster of
-// that size, "0" none.
+// (0: none -- the level-by-level path runs).  By default an 8-CTA cluster takes
+// the levels of at most CC_ROWS rows, and of at most CC_BLOCK_ROWS where the
+// level's sweeps can run by blocks (sell.cu).  Measured: a level of 4,913 rows
+// (Q2 8^3) in the cluster 0.29 ms per V-cycle more than by blocks (FP64 V-cycle
+// of the 32^3 Q2 hierarchy 1.25 against 0.95 ms; Q1 32^3 Poisson solve 2.99
+// against 1.99 ms), one of 729 rows 0.02 ms less; without blocks the colour
+// launches are the alternative (64^3 Q2 FP32 V-cycle 4.31 ms against 4.17 ms with
+// the levels of at most 8192 rows in the cluster; larger levels stream more
+// matrix per colour pass than one GPC's share of L2 bandwidth carries).
+// PMG_COARSE_CLUSTER=<ctas>[:<max rows>] chooses another shape: "8:8192" the
+// levels of at most 8192 rows on an 8-CTA cluster whether or not they have
+// blocks, "1" the levels of at most CC_ONE_CTA_ROWS rows on one CTA, "16" (2, 4,
+// 8) every level whose iterates fit CC_SMEM_X on a cluster of that size, "0" none.
+constexpr int CC_ROWS = 8192, CC_BLOCK_ROWS = 2000;
 constexpr int CC_ONE_CTA_ROWS = 8192;
 
 int coarse_cycle_top(Handle &h) {
   static int mode = -1;  // 0 off, 1 one CTA, 2 cluster
-  static long max_rows = 0;
+  static long max_rows = 0, max_block_rows = 0;
   static int want = 0;   // CTAs asked for
   if (mode < 0) {
     const char *e = getenv("PMG_COARSE_CLUSTER");
-    const std::string v(e ? e : "8:8192");
+    const std::string v(e ? e : "8:" + std::to_string(CC_ROWS));
     const size_t colon = v.find(':');
     want = atoi(v.substr(0, colon).c_str());
     mode = want == 1 ? 1 : (want == 2 || want == 4 || want == 8 || want == 16) ? 2 : 0;
     max_rows = mode == 1 ? CC_ONE_CTA_ROWS : 0;
     if (mode && colon != std::string::npos) max_rows = atol(v.c_str() + colon + 1);
+    max_block_rows = e ? max_rows : CC_BLOCK_ROWS;
   }
   if (mode == 0) return 0;
   // the one-launch cycle runs SSOR pre/post steps without step-length control
@@ -561,14 +568,10 @@ int coarse_cycle_top(Handle &h) {
     const Level &L = h.lv[i];
     bytes += ((size_t)L.N * vb + 15) / 16 * 16;
     if (bytes > CC_SMEM_X || (int)L.sell_group.size() > CC_MAX_GROUPS) break;
-    if (max_rows > 0 && L.N > max_rows) break;
+    if (max_rows > 0 && L.N > (L.blk_col.empty() ? max_rows : max_block_rows)) break;
     top = i;
   }
   if (top < 1) return 0;
-  if (!h.cc_err.p) {
-    if (h.cc_err.alloc(1) != PMG_OK) return 0;
-    if (cudaMemset(h.cc_err.p, 0, sizeof(int)) != cudaSuccess) return 0;
-  }
   if (mode == 1) {
     h.cc_ctas = 1;
   } else {
@@ -581,12 +584,11 @@ int coarse_cycle_top(Handle &h) {
 }
 
 int coarse_cycle_check(Handle &h) {
-  if (!h.cc_err.p) return PMG_OK;
   int e = 0;
   PMG_CUDA(cudaMemcpy(&e, h.cc_err.p, sizeof(int), cudaMemcpyDeviceToHost));
   if (!e) return PMG_OK;
   PMG_CUDA(cudaMemset(h.cc_err.p, 0, sizeof(int)));
-  set_error("coarse cycle: a cluster wait gave up (updates of a pass never arrived)");
+  set_error("V-cycle: a bounded wait of the coarse cycle or of a block sweep gave up (updates of a pass never arrived)");
   return PMG_ERR_STATE;
 }
 

@@ -221,6 +221,8 @@ int pmg_create(pmg_handle *out, int n_levels, const pmg_params *p) {
     if (cudaEventCreateWithFlags(&h->aux_ev[k], cudaEventDisableTiming) != cudaSuccess) rc = PMG_ERR_CUDA;
   if (rc == PMG_OK) rc = h->coarse_flags.alloc(4);
   if (rc == PMG_OK && cudaMallocHost(&h->h_coarse_flags, sizeof(int) * 4) != cudaSuccess) rc = PMG_ERR_CUDA;
+  if (rc == PMG_OK) rc = h->cc_err.alloc(1);
+  if (rc == PMG_OK && cudaMemset(h->cc_err.p, 0, sizeof(int)) != cudaSuccess) rc = PMG_ERR_CUDA;
   if (rc == PMG_OK) rc = h->red_partial.alloc(1024);
   if (rc == PMG_OK) rc = h->red_counter.alloc(1);
   if (rc == PMG_OK && cudaMemset(h->red_counter.p, 0, sizeof(unsigned)) != cudaSuccess) rc = PMG_ERR_CUDA;
@@ -720,8 +722,8 @@ int pmg_time_kernel(pmg_handle hh, int kernel, int level, int form, int reps, do
     switch (kernel) {
       case PMG_KERNEL_SPMV64: return sell_spmv<double>(s, L, x64.p, nullptr, y64.p, 0, h->num_sms);
       case PMG_KERNEL_SPMV32: return sell_spmv<float>(s, L, x32.p, nullptr, y32.p, 0, h->num_sms);
-      case PMG_KERNEL_SSOR64: return sell_ssor<double>(s, L, y64.p, x64.p, 1.0, h->num_sms);
-      case PMG_KERNEL_SSOR32: return sell_ssor<float>(s, L, y32.p, x32.p, 1.0, h->num_sms);
+      case PMG_KERNEL_SSOR64: return sell_ssor<double>(s, L, y64.p, x64.p, 1.0, h->num_sms, 1, SWEEP_ANY, h->cc_err.p);
+      case PMG_KERNEL_SSOR32: return sell_ssor<float>(s, L, y32.p, x32.p, 1.0, h->num_sms, 1, SWEEP_ANY, h->cc_err.p);
       case PMG_KERNEL_CSR_SPMV64: return spmv<double>(s, L, L.A.p, x64.p, y64.p);
       case PMG_KERNEL_ASSEMBLE: return assemble_level(*h, L, form, L.A.p, true, L.rhs.p);
       case PMG_KERNEL_COARSE_FACTOR: return coarse_factor(*h);
@@ -739,7 +741,11 @@ int pmg_time_kernel(pmg_handle hh, int kernel, int level, int form, int reps, do
       spmv_b = 8.0 * (L.sell_nnz_narrow + L.sell_nnz_wide) + 2.0 * L.sell_nnz_narrow + 4.0 * L.sell_nnz_wide +
                4.0 * (L.sell_nslices + 1) + 4 * N + 16 * N;
     }
-    by = kernel == PMG_KERNEL_SSOR64 ? 2 * spmv_b + 16 * N : spmv_b;
+    // an SSOR step on an arbitrary x: forward over whole rows, backward over their
+    // upper halves (whole rows again when the pattern is not split)
+    by = spmv_b;
+    if (kernel == PMG_KERNEL_SSOR64)
+      by += spmv_b + 16 * N - (L.sell_split ? 0.5 * (10.0 * L.sell_nnz_narrow + 12.0 * L.sell_nnz_wide) : 0.0);
     fl = kernel == PMG_KERNEL_SSOR64 ? 4 * nnz : 2 * nnz;
   } else if (kernel == PMG_KERNEL_SPMV32 || kernel == PMG_KERNEL_SSOR32) {
     PMG_TRY(sell_values<float>(*h, L));
@@ -748,7 +754,9 @@ int pmg_time_kernel(pmg_handle hh, int kernel, int level, int form, int reps, do
     PMG_CUDA(cudaMemsetAsync(y32.p, 0, sizeof(float) * L.N, s));
     double spmv_b = 4.0 * (L.sell_nnz_narrow + L.sell_nnz_wide) + 2.0 * L.sell_nnz_narrow + 4.0 * L.sell_nnz_wide +
                     4.0 * (L.sell_nslices + 1) + 4 * N + 8 * N;
-    by = kernel == PMG_KERNEL_SPMV32 ? spmv_b : 2 * spmv_b + 8 * N;
+    by = spmv_b;
+    if (kernel == PMG_KERNEL_SSOR32)
+      by += spmv_b + 8 * N - (L.sell_split ? 0.5 * (6.0 * L.sell_nnz_narrow + 8.0 * L.sell_nnz_wide) : 0.0);
     fl = kernel == PMG_KERNEL_SPMV32 ? 2 * nnz : 4 * nnz;
   } else if (kernel == PMG_KERNEL_COARSE_FACTOR) {
     if (level != 0) { set_error("pmg_time_kernel: the coarse factorisation is of level 0"); return PMG_ERR_ARG; }

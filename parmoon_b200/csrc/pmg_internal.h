@@ -97,6 +97,8 @@ struct ElemInfo {
 };
 ElemInfo elem_info(int elem_type);
 
+constexpr int SELL_NO_SRC = 65535;
+
 // one multigrid level
 struct Level {
   // sizes
@@ -162,6 +164,28 @@ struct Level {
   DBuf<int> sell_alen;           // entries of each row in the solve copy
   DBuf<int> dd_row, dd_beg;      // active rows with Dirichlet columns, first such CSR position
   int n_dd = 0;
+  // the rows' entries split by colour: steps [0, nlow) of a slice hold the
+  // columns of lower colours, step nlow the diagonal, the rest the higher
+  // ones; sell_src: an entry's position in its CSR row (SELL_NO_SRC: padding)
+  bool sell_split = false;
+  DBuf<int> sell_nlow;
+  DBuf<unsigned short> sell_src;
+  DBuf<float> sell_sl32, sell_su32;  // sums over the lower / higher colours kept between sweeps
+  DBuf<double> sell_sl64, sell_su64;
+  // phases and blocks of the sweeps (sell.cu, find_blocks): phase p holds the
+  // colours [blk_col[p], blk_col[p + 1]); its rows fall into blk_n[p] blocks
+  // that are not coupled inside the phase.  sell_in: a slice's steps in its own
+  // block next to the diagonal (lower | upper << 16); sell_loc: their columns as
+  // slots of the block.  blk_tab from blk_tab0[p]: per block its first slice in
+  // blk_meta / blk_rows, the first ordinal of every colour, the number of slices
+  std::vector<int> blk_col, blk_n, blk_tab0, blk_slots;
+  DBuf<int> blk_tab, blk_meta, blk_rows, sell_in;
+  DBuf<unsigned short> sell_loc;
+  long blk_chunks = 0;         // chunks of 4 steps of the inside entries
+  DBuf<float> blk_val32;       // their values in that layout
+  DBuf<double> blk_val64;
+  DBuf<float> sell_base32;   // f minus the sums from outside the block (slice order)
+  DBuf<double> sell_base64;
   long sell_nnz_narrow = 0, sell_nnz_wide = 0;  // stored entries with 16-bit / 32-bit columns
   DBuf<float> sell_val32, sell_invd32;
   DBuf<double> sell_val64, sell_invd64;
@@ -298,12 +322,18 @@ template <typename T>
 int sell_values(Handle &h, Level &L);
 template <typename T>
 int sell_spmv(cudaStream_t s, const Level &L, const T *x, const T *f, T *y, int mode, int num_sms);
+// what is known of x when SSOR steps start: nothing, or x = 0 on the active rows
+enum SweepStart { SWEEP_ANY, SWEEP_ZERO };
+// `steps` SSOR steps on the active rows (x_D = f_D holds already); err: Handle::cc_err
 template <typename T>
-int sell_ssor(cudaStream_t s, const Level &L, const T *f, T *x, double omega, int num_sms, bool dirichlet = true,
-              bool after_ssor = false, bool skip_repeats = false, bool forward_only = false);
+int sell_ssor(cudaStream_t s, const Level &L, const T *f, T *x, double omega, int num_sms, int steps, SweepStart start,
+              int *err);
+// one SOR step (forward sweep) on the active rows
+template <typename T>
+int sell_sor(cudaStream_t s, const Level &L, const T *f, T *x, double omega, int num_sms);
 // one damped Jacobi step; tmp: a level-sized work vector other than x and f
 template <typename T>
-int sell_jacobi(cudaStream_t s, const Level &L, const T *f, T *x, T *tmp, double omega, int num_sms, bool dirichlet);
+int sell_jacobi(cudaStream_t s, const Level &L, const T *f, T *x, T *tmp, double omega, int num_sms);
 // y_a -= A_aD v_D (add: y_a += A_aD v_D) over the active rows' Dirichlet
 // columns (the part of A the solve copy leaves out)
 template <typename T>

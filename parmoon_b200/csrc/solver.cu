@@ -379,21 +379,28 @@ template <> struct Prec<float> {
   static float *jac(Level &L) { return L.jac32.p; }
 };
 
-// one pre/post smoothing step (TMultiGrid3D::Smooth, MultiGrid3D.C:117-446):
-// Jacobi, SOR or SSOR in colour order (kind = PMG_SMOOTHER_*), or
-// x += omega W (f - A x) with the learned stencil
+// `steps` pre/post smoothing steps (TMultiGrid3D::Smooth, MultiGrid3D.C:117-446):
+// Jacobi, SOR or SSOR in colour order (params.smoother), or x += omega W (f - A x)
+// with the learned stencil.  x_D = f_D holds already: k_prec_in32 / 64 set it on
+// the finest level, and on the coarser ones the restriction writes 0 into both.
 template <typename T>
-static int smooth_step(Handle &h, Level &L, bool learned, bool first, bool after_ssor, int kind) {
+static int smooth(Handle &h, Level &L, bool learned, int steps, SweepStart start) {
   using PT = Prec<T>;
-  if (learned) {
-    PMG_TRY(sell_spmv<T>(h.stream, L, PT::x(L), PT::f(L), PT::d(L), 1, h.num_sms));
-    return learned_smooth<T>(h.stream, L, PT::d(L), PT::x(L), h.prm.smooth_omega);
+  const int kind = h.prm.smoother;
+  if (!learned && kind != PMG_SMOOTHER_JACOBI && kind != PMG_SMOOTHER_SOR)
+    return sell_ssor<T>(h.stream, L, PT::f(L), PT::x(L), h.prm.smooth_omega, h.num_sms, steps, start,
+                        h.cc_err.p);
+  for (int k = 0; k < steps; k++) {
+    if (learned) {
+      PMG_TRY(sell_spmv<T>(h.stream, L, PT::x(L), PT::f(L), PT::d(L), 1, h.num_sms));
+      PMG_TRY(learned_smooth<T>(h.stream, L, PT::d(L), PT::x(L), h.prm.smooth_omega));
+    } else if (kind == PMG_SMOOTHER_JACOBI) {
+      PMG_TRY(sell_jacobi<T>(h.stream, L, PT::f(L), PT::x(L), PT::jac(L), h.prm.smooth_omega, h.num_sms));
+    } else {
+      PMG_TRY(sell_sor<T>(h.stream, L, PT::f(L), PT::x(L), h.prm.smooth_omega, h.num_sms));
+    }
   }
-  if (kind == PMG_SMOOTHER_JACOBI)
-    return sell_jacobi<T>(h.stream, L, PT::f(L), PT::x(L), PT::jac(L), h.prm.smooth_omega, h.num_sms, first);
-  if (kind == PMG_SMOOTHER_SOR)
-    return sell_ssor<T>(h.stream, L, PT::f(L), PT::x(L), h.prm.smooth_omega, h.num_sms, first, false, false, true);
-  return sell_ssor<T>(h.stream, L, PT::f(L), PT::x(L), h.prm.smooth_omega, h.num_sms, first, after_ssor, true);
+  return PMG_OK;
 }
 
 // Step-length control (TMGLevel3D::StepLengthControl, MGLevel3D.C:908-961,
@@ -612,13 +619,15 @@ static int vcycle(Handle &h, int i, bool learned) {
   const int post = (learned && h.prm.learned_steps > 0) ? h.prm.learned_steps : h.prm.post_smooth;
   const bool slc = h.prm.slc_all || (h.prm.slc_fine && i == (int)h.lv.size() - 1);
   if (slc) PMG_TRY(slc_begin<T>(h, L));
-  for (int k = 0; k < pre; k++) PMG_TRY(smooth_step<T>(h, L, learned, k == 0, k > 0, h.prm.smoother));
-  PMG_TRY(sell_spmv<T>(s, L, PT::x(L), PT::f(L), PT::d(L), 1, h.num_sms));
+  PMG_TRY(smooth<T>(h, L, learned, pre, SWEEP_ZERO));
+  // after SSOR steps the defect needs one side of the matrix only
+  const bool half = !learned && pre > 0 && h.prm.smoother != PMG_SMOOTHER_JACOBI &&
+                    h.prm.smoother != PMG_SMOOTHER_SOR && L.sell_split;
+  PMG_TRY(sell_spmv<T>(s, L, PT::x(L), PT::f(L), PT::d(L), half ? 3 : 1, h.num_sms));
   PMG_TRY(restrict_defect<T>(s, L, C, PT::R(L), PT::d(L), PT::f(C), PT::x(C)));  // also x_C := 0
   PMG_TRY(vcycle<T>(h, i - 1, learned));
   PMG_TRY(prolongate_add<T>(s, L, PT::P(L), PT::x(C), PT::x(L), h.prm.gmg_damp));
-  for (int k = 0; k < post; k++)
-    PMG_TRY(smooth_step<T>(h, L, learned, pre == 0 && k == 0, k > 0, h.prm.smoother));
+  PMG_TRY(smooth<T>(h, L, learned, post, SWEEP_ANY));
   if (slc) PMG_TRY(slc_end<T>(h, L));
   return PMG_OK;
 }
