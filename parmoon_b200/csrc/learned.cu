@@ -14,14 +14,16 @@
 // activations (every layer's input is rounded to BF16), FP32 accumulation.
 // The forward runs on the tensor cores as an implicit GEMM per brick of the
 // lattice (mma.sync m16n8k16 BF16: rows = nodes, columns = output channels,
-// reduction = 27 offsets x 32 input channels); the backward (data and weight
-// gradients) and Adam run on FP32 CUDA cores.  Training runs on the device
-// through the pmg_learned_* entry points.
+// reduction = 27 offsets x 32 input channels), and so does the backward: the
+// activations and weights it multiplies with are BF16 already, and an FP32
+// gradient is the sum of three BF16 numbers (its leading 8 bits, the next 8, the
+// rest), so three BF16 products with FP32 accumulation give the FP32 product.
+// Adam runs on FP32.  Training runs on the device through the pmg_learned_*
+// entry points.
 //
-// Lattice order: node L = i + n1 (j + n1 k).  The forward's activations are
-// node-major BF16 with the channels padded to 32 (L * 32 + c); the FP32
-// arrays of the backward are channel-major (c * NL + L).  Offsets:
-// k = (di+1) + 3 (dj+1) + 9 (dk+1).
+// Lattice order: node L = i + n1 (j + n1 k).  Activations are node-major BF16
+// with the channels padded to 32 (L * 32 + c); gradients likewise, three such
+// arrays one after the other.  Offsets: k = (di+1) + 3 (dj+1) + 9 (dk+1).
 #include "pmg_internal.h"
 #include <cuda_bf16.h>
 #include <cmath>
@@ -45,14 +47,12 @@ __device__ __forceinline__ int lat_nb(int L, int k, int n1) {
 
 // ------------------------------------------------------------- features
 // feature k of node L = a(i, nb_k(i)) / a(i,i) for an active row i at node L
-// (0 elsewhere), rounded to BF16: xf[L * 32 + k] (channels 27..31 stay 0) and,
-// when feat != NULL (training), the same values FP32 channel-major;
+// (0 elsewhere), rounded to BF16: xf[L * 32 + k] (channels 27..31 stay 0);
 // dscale[L] = 1 / a(i,i) for active rows, 0 for Dirichlet rows.  The caller
-// zeroes xf (and feat).
+// zeroes xf.
 __global__ void k_features(int N, int Na, int n1, const int *__restrict__ rp, const int *__restrict__ kc,
                            const double *__restrict__ a, const int *__restrict__ dof_lat, __nv_bfloat16 *__restrict__ xf,
-                           float *__restrict__ feat, float *__restrict__ dscale) {
-  const int NL = n1 * n1 * n1;
+                           float *__restrict__ dscale) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= N) return;
   const int L = dof_lat[r];
@@ -65,9 +65,7 @@ __global__ void k_features(int N, int Na, int n1, const int *__restrict__ rp, co
     const int di = Lc % n1 - i, dj = (Lc / n1) % n1 - j, dk = Lc / (n1 * n1) - kk;
     if (di < -1 || di > 1 || dj < -1 || dj > 1 || dk < -1 || dk > 1) continue;  // not on a 27-point stencil
     const int k = (di + 1) + 3 * (dj + 1) + 9 * (dk + 1);
-    const __nv_bfloat16 v = __float2bfloat16((float)(a[p] / diag));
-    xf[(size_t)L * 32 + k] = v;
-    if (feat) feat[(size_t)k * NL + L] = __bfloat162float(v);
+    xf[(size_t)L * 32 + k] = __float2bfloat16((float)(a[p] / diag));
   }
   dscale[L] = (float)(1.0 / diag);
 }
@@ -79,6 +77,25 @@ __global__ void k_pack_weights(int cin, int cout, const __nv_bfloat16 *__restric
   if (t >= 27 * 32 * 32) return;
   const int k = t >> 10, co = (t >> 5) & 31, ci = t & 31;
   wpk[t] = (co < cout && ci < cin) ? w[((size_t)co * cin + ci) * 27 + k] : __float2bfloat16(0.0f);
+}
+
+// The same for the data gradient, whose input channels are the layer's outputs:
+// dx[ci][L] = sum_{co,k} w[co][ci][k] dz[co][L - o_k] is a convolution with the
+// offsets reversed (-o_k = o_{26-k}) and the channels exchanged.
+__global__ void k_pack_weights_t(int cin, int cout, const __nv_bfloat16 *__restrict__ w,
+                                 __nv_bfloat16 *__restrict__ wpk) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 27 * 32 * 32) return;
+  const int k = t >> 10, ci = (t >> 5) & 31, co = t & 31;
+  wpk[t] = (co < cout && ci < cin) ? w[((size_t)co * cin + ci) * 27 + 26 - k] : __float2bfloat16(0.0f);
+}
+
+// v = h + m + l, three BF16 numbers (exact: 3 x 8 significant bits, up to underflow)
+__device__ __forceinline__ void split3(float v, __nv_bfloat16 &h, __nv_bfloat16 &m, __nv_bfloat16 &l) {
+  h = __float2bfloat16(v);
+  const float r = v - __bfloat162float(h);
+  m = __float2bfloat16(r);
+  l = __float2bfloat16(r - __bfloat162float(m));
 }
 
 // ------------------------------------------------------------- tensor-core convolution
@@ -117,15 +134,19 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// LAST = false: out = ReLU(conv + b) as BF16 node-major into xo; with a_cm /
-//   z_cm (training) also the rounded activation and the pre-activation, FP32
-//   channel-major.
-// LAST = true: the stencil W[co][L] = (conv + b)[co] * dscale[L], co < cout.
-template <bool LAST>
+// CONV_HIDDEN: xo = ReLU(conv + b) as BF16.
+// CONV_STENCIL: the stencil W[co][L] = (conv + b)[co] * dscale[L], co < cout.
+// CONV_GRAD: the data gradient: the input is a gradient in three BF16 parts
+//   (accumulated one after the other), xo gets conv * (act > 0) in three parts, and
+//   bsum[CTA][32] the CTA's sums of it per channel (the bias gradient's partials).
+//   0.22 ms per 32 x 32 layer at 65^3 nodes (FP32 CUDA cores before: 0.81 ms).
+enum { CONV_HIDDEN = 0, CONV_STENCIL = 1, CONV_GRAD = 2 };
+template <int MODE>
 __global__ void __launch_bounds__(256, 2)
     k_conv_tc(int n1, int cout, const __nv_bfloat16 *__restrict__ xi, const __nv_bfloat16 *__restrict__ wpk,
-              const __nv_bfloat16 *__restrict__ bias, __nv_bfloat16 *__restrict__ xo, float *__restrict__ a_cm,
-              float *__restrict__ z_cm, const float *__restrict__ dscale, float *__restrict__ Wst) {
+              const __nv_bfloat16 *__restrict__ bias, __nv_bfloat16 *__restrict__ xo, const float *__restrict__ dscale,
+              float *__restrict__ Wst, const __nv_bfloat16 *__restrict__ act, float *__restrict__ bsum) {
+  constexpr bool LAST = MODE == CONV_STENCIL, GRAD = MODE == CONV_GRAD;
   extern __shared__ __align__(128) unsigned char conv_sm[];
   const unsigned s_halo = (unsigned)__cvta_generic_to_shared(conv_sm);
   const unsigned s_w = s_halo + CONV_HALO * 64;
@@ -137,13 +158,14 @@ __global__ void __launch_bounds__(256, 2)
     const uint4 v = __ldg(reinterpret_cast<const uint4 *>(wpk) + t);
     *reinterpret_cast<uint4 *>(conv_sm + CONV_HALO * 64 + swz(row, ch)) = v;
   }
-  float bv[4][2];
+  float bv[4][2], bs[4][2];
 #pragma unroll
   for (int nt = 0; nt < 4; nt++)
 #pragma unroll
     for (int e = 0; e < 2; e++) {
       const int co = nt * 8 + 2 * (lane & 3) + e;
-      bv[nt][e] = co < cout ? __bfloat162float(bias[co]) : 0.0f;
+      bv[nt][e] = !GRAD && co < cout ? __bfloat162float(bias[co]) : 0.0f;
+      bs[nt][e] = 0.0f;
     }
   const int nbx = (n1 + CONV_BX - 1) / CONV_BX, nby = (n1 + CONV_BY - 1) / CONV_BY, nbz = (n1 + CONV_BZ - 1) / CONV_BZ;
   const int nbricks = nbx * nby * nbz;
@@ -154,19 +176,6 @@ __global__ void __launch_bounds__(256, 2)
   for (int br = blockIdx.x; br < nbricks; br += gridDim.x) {
     const int bx = br % nbx, by = (br / nbx) % nby, bz = br / (nbx * nby);
     const int x0 = bx * CONV_BX, y0 = by * CONV_BY, z0 = bz * CONV_BZ;
-    __syncthreads();  // the previous brick's reads of the halo are done
-    for (int t = tid; t < CONV_HALO * 4; t += blockDim.x) {
-      const int node = t >> 2, ch = t & 3;
-      const int hx = node % CONV_HX, hy = (node / CONV_HX) % CONV_HY, hz = node / (CONV_HX * CONV_HY);
-      const int gx = x0 - 1 + hx, gy = y0 - 1 + hy, gz = z0 - 1 + hz;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (gx >= 0 && gy >= 0 && gz >= 0 && gx < n1 && gy < n1 && gz < n1) {
-        const size_t L = (size_t)gx + (size_t)n1 * ((size_t)gy + (size_t)n1 * gz);
-        v = __ldg(reinterpret_cast<const uint4 *>(xi + L * 32) + ch);
-      }
-      *reinterpret_cast<uint4 *>(conv_sm + swz(node, ch)) = v;
-    }
-    __syncthreads();
     float acc[2][4][4];
 #pragma unroll
     for (int m = 0; m < 2; m++)
@@ -174,29 +183,47 @@ __global__ void __launch_bounds__(256, 2)
       for (int nt = 0; nt < 4; nt++)
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[m][nt][e] = 0.0f;
+    // (the smallest part first: the tensor cores round every sum towards zero, and
+    // relative to a small sum that is little)
+    for (int part = GRAD ? 2 : 0; part >= 0; part--) {
+      const __nv_bfloat16 *xp = xi + part * NL * 32;
+      __syncthreads();  // the previous reads of the halo are done
+      for (int t = tid; t < CONV_HALO * 4; t += blockDim.x) {
+        const int node = t >> 2, ch = t & 3;
+        const int hx = node % CONV_HX, hy = (node / CONV_HX) % CONV_HY, hz = node / (CONV_HX * CONV_HY);
+        const int gx = x0 - 1 + hx, gy = y0 - 1 + hy, gz = z0 - 1 + hz;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (gx >= 0 && gy >= 0 && gz >= 0 && gx < n1 && gy < n1 && gz < n1) {
+          const size_t L = (size_t)gx + (size_t)n1 * ((size_t)gy + (size_t)n1 * gz);
+          v = __ldg(reinterpret_cast<const uint4 *>(xp + L * 32) + ch);
+        }
+        *reinterpret_cast<uint4 *>(conv_sm + swz(node, ch)) = v;
+      }
+      __syncthreads();
 #pragma unroll 3
-    for (int k = 0; k < 27; k++) {
-      const int dx = k % 3, dy = (k / 3) % 3, dz = k / 9;
+      for (int k = 0; k < 27; k++) {
+        const int dx = k % 3, dy = (k / 3) % 3, dz = k / 9;
 #pragma unroll
-      for (int kc = 0; kc < 2; kc++) {
-        unsigned a[2][4], b[2][4];
+        for (int kc = 0; kc < 2; kc++) {
+          unsigned a[2][4], b[2][4];
 #pragma unroll
-        for (int m = 0; m < 2; m++) {
-          const int row = (a_row + dx) + CONV_HX * ((warp + dy) + CONV_HY * (m + dz));
-          ldsm_x4(s_halo + swz(row, 2 * kc + a_half), a[m]);
-        }
-#pragma unroll
-        for (int p = 0; p < 2; p++) {
-          const int row = k * 32 + 16 * p + b_co;
-          ldsm_x4(s_w + swz(row, 2 * kc + b_half), b[p]);
-        }
-#pragma unroll
-        for (int m = 0; m < 2; m++)
+          for (int m = 0; m < 2; m++) {
+            const int row = (a_row + dx) + CONV_HX * ((warp + dy) + CONV_HY * (m + dz));
+            ldsm_x4(s_halo + swz(row, 2 * kc + a_half), a[m]);
+          }
 #pragma unroll
           for (int p = 0; p < 2; p++) {
-            mma_bf16(acc[m][2 * p], a[m], b[p][0], b[p][1]);
-            mma_bf16(acc[m][2 * p + 1], a[m], b[p][2], b[p][3]);
+            const int row = k * 32 + 16 * p + b_co;
+            ldsm_x4(s_w + swz(row, 2 * kc + b_half), b[p]);
           }
+#pragma unroll
+          for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+              mma_bf16(acc[m][2 * p], a[m], b[p][0], b[p][1]);
+              mma_bf16(acc[m][2 * p + 1], a[m], b[p][2], b[p][3]);
+            }
+        }
       }
     }
     // epilogue: c0,c1 = (row g, channels 2q, 2q+1), c2,c3 = (row g+8, ...)
@@ -214,105 +241,210 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
         for (int nt = 0; nt < 4; nt++) {
           const int co = nt * 8 + 2 * q;
-          const float v0 = acc[m][nt][2 * hrow] + bv[nt][0], v1 = acc[m][nt][2 * hrow + 1] + bv[nt][1];
+          float v0 = acc[m][nt][2 * hrow] + bv[nt][0], v1 = acc[m][nt][2 * hrow + 1] + bv[nt][1];
           if (LAST) {
             if (co < cout) Wst[(size_t)co * NL + L] = v0 * ds;
             if (co + 1 < cout) Wst[(size_t)(co + 1) * NL + L] = v1 * ds;
+          } else if (GRAD) {
+            const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162 *>(act + L * 32 + co);
+            if (!(__low2float(x) > 0.0f)) v0 = 0.0f;
+            if (!(__high2float(x) > 0.0f)) v1 = 0.0f;
+            bs[nt][0] += v0;
+            bs[nt][1] += v1;
+            __nv_bfloat162 h, mi, l;
+            split3(v0, h.x, mi.x, l.x);
+            split3(v1, h.y, mi.y, l.y);
+            *reinterpret_cast<__nv_bfloat162 *>(xo + L * 32 + co) = h;
+            *reinterpret_cast<__nv_bfloat162 *>(xo + (NL + L) * 32 + co) = mi;
+            *reinterpret_cast<__nv_bfloat162 *>(xo + (2 * NL + L) * 32 + co) = l;
           } else {
-            const __nv_bfloat162 r = __floats2bfloat162_rn(fmaxf(v0, 0.0f), fmaxf(v1, 0.0f));
-            *reinterpret_cast<__nv_bfloat162 *>(xo + L * 32 + co) = r;
-            if (a_cm) {
-              a_cm[(size_t)co * NL + L] = __low2float(r);
-              a_cm[(size_t)(co + 1) * NL + L] = __high2float(r);
-              z_cm[(size_t)co * NL + L] = v0;
-              z_cm[(size_t)(co + 1) * NL + L] = v1;
-            }
+            *reinterpret_cast<__nv_bfloat162 *>(xo + L * 32 + co) =
+                __floats2bfloat162_rn(fmaxf(v0, 0.0f), fmaxf(v1, 0.0f));
           }
         }
       }
     }
   }
-}
-
-// dx[ci][L] = sum_{co,k} w[co][ci][k] dz[co][L - o_k]  (neighbour L' with nb_k(L') = L)
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_conv_bwd_data(int n1, const float *__restrict__ dz, const __nv_bfloat16 *__restrict__ w,
-                                                       float *__restrict__ dx) {
-  extern __shared__ float sw[];  // [co][k][ci]
-  const int NL = n1 * n1 * n1;
-  for (int t = threadIdx.x; t < COUT * CIN * 27; t += blockDim.x) {
-    const int co = t / (CIN * 27), rem = t % (CIN * 27);
-    const int ci = rem / 27, k = rem % 27;
-    sw[(co * 27 + k) * CIN + ci] = __bfloat162float(w[t]);
-  }
-  __syncthreads();
-  const int L = blockIdx.x * blockDim.x + threadIdx.x;
-  if (L >= NL) return;
-  float acc[CIN];
-#pragma unroll
-  for (int ci = 0; ci < CIN; ci++) acc[ci] = 0.0f;
-  for (int k = 0; k < 27; k++) {
-    const int src = lat_nb(L, 26 - k, n1);  // L - o_k
-    if (src < 0) continue;
-    for (int co = 0; co < COUT; co++) {
-      const float g = dz[(size_t)co * NL + src];
-      const float *wr = sw + (co * 27 + k) * CIN;
-#pragma unroll
-      for (int ci = 0; ci < CIN; ci++) acc[ci] += wr[ci] * g;
-    }
-  }
-#pragma unroll
-  for (int ci = 0; ci < CIN; ci++) dx[(size_t)ci * NL + L] = acc[ci];
-}
-
-// gw[co][ci][k] += sum_L dz[co][L] x[ci][nb_k(L)] ; gb[co] += sum_L dz[co][L]
-// one block per (ci, k); threads stride over L with COUT accumulators
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) k_conv_bwd_weight(int n1, const float *__restrict__ dz, const float *__restrict__ x,
-                                                         float *__restrict__ gw, float *__restrict__ gb) {
-  const int NL = n1 * n1 * n1;
-  const int ci = blockIdx.x / 27, k = blockIdx.x % 27;
-  const bool do_bias = (blockIdx.x == 0);
-  float acc[COUT], accb[COUT];
-#pragma unroll
-  for (int co = 0; co < COUT; co++) { acc[co] = 0.0f; accb[co] = 0.0f; }
-  for (int L = threadIdx.x; L < NL; L += blockDim.x) {
-    const int nb = lat_nb(L, k, n1);
-    const float xv = nb >= 0 ? x[(size_t)ci * NL + nb] : 0.0f;
-#pragma unroll
-    for (int co = 0; co < COUT; co++) {
-      const float g = dz[(size_t)co * NL + L];
-      acc[co] += g * xv;
-      if (do_bias) accb[co] += g;
-    }
-  }
-  __shared__ float red[256];
-  for (int co = 0; co < COUT; co++) {
-    red[threadIdx.x] = acc[co];
+  if (GRAD) {
+    // per channel: over the lanes of equal q, then over the warps
     __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-      if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) gw[(size_t)(co * CIN + ci) * 27 + k] += red[0];
-    __syncthreads();
-    if (do_bias) {
-      red[threadIdx.x] = accb[co];
-      __syncthreads();
-      for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
+    float *sb = reinterpret_cast<float *>(conv_sm);
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        float v = bs[nt][e];
+        for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane < 4) sb[warp * 32 + nt * 8 + 2 * lane + e] = v;
       }
-      if (threadIdx.x == 0) gb[co] += red[0];
-      __syncthreads();
+    __syncthreads();
+    if (tid < 32) {
+      float v = 0.0f;
+      for (int w = 0; w < 8; w++) v += sb[w * 32 + tid];
+      bsum[blockIdx.x * 32 + tid] = v;
     }
   }
 }
 
-// ReLU backward in place: g = g * (z > 0)
-__global__ void k_relu_bwd(size_t n, const float *__restrict__ z, float *__restrict__ g) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    if (!(z[i] > 0.0f)) g[i] = 0.0f;
+// ------------------------------------------------------------- weight gradient
+// gw[co][ci][k] = sum_L dz[co][L] x[ci][L + o_k] as 27 products 32 x NL x 32 on the
+// tensor cores: the reduction runs over the nodes, so both operands are read
+// transposed (ldmatrix.trans) from their node-major bricks -- dz (three BF16
+// parts) of 16 x 8 nodes and x with its one-node halo -- in shared memory, the
+// next brick on its way by cp.async meanwhile.  18 warps: warp w holds the
+// accumulators of offsets 3 (w % 9) .. + 2 for 16 of the 32 channels co; per 16
+// nodes 3 + 6 ldmatrix.x4 feed 36 mma.  The tensor cores round their sums towards
+// zero, so after every WG_FLUSH runs of 16 nodes (6 mma) a thread adds its accumulators
+// to FP32 sums of its own in shared memory and starts from 0 again.  One CTA per
+// SM; every CTA leaves its sums in part[CTA] and k_wgrad_sum adds those in order,
+// so the result does not depend on the schedule.
+// At 65^3 nodes 0.20 ms per layer (46 GFLOP in three parts, bound by the mma.sync
+// and ldmatrix issue rate); the FP32 kernel before it read dz once per (ci, k)
+// through L2, 864 times in all, and took 5.4 ms.  Against FP64 the gradient is
+// as far off as with that kernel (1.0002 times on average over lattices of 9 to
+// 65 nodes a side; without taking the sums out 1.06 times at 65).
+constexpr int WG_WARPS = 18, WG_NODES = CONV_BX * CONV_BY, WG_HALO = CONV_HX * CONV_HY * 3, WG_FLUSH = 2;
+constexpr int WG_STAGE = (WG_HALO + 3 * WG_NODES) * 64;  // 59,136 bytes, two stages
+constexpr int WG_SMEM = 2 * WG_STAGE + 48 * 32 * WG_WARPS * (int)sizeof(float);
+__device__ __forceinline__ void ldsm_x4_t(unsigned addr, unsigned (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void cp_async16(unsigned dst, const void *src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(32 * WG_WARPS, 1)
+    k_conv_wgrad(int n1, const __nv_bfloat16 *__restrict__ dz, const __nv_bfloat16 *__restrict__ x,
+                 float *__restrict__ part) {
+  extern __shared__ __align__(128) unsigned char conv_sm[];
+  const unsigned sm = (unsigned)__cvta_generic_to_shared(conv_sm);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wo = warp % 9, mt = warp / 9;
+  const size_t NL = (size_t)n1 * n1 * n1;
+  const int nbx = (n1 + CONV_BX - 1) / CONV_BX, nby = (n1 + CONV_BY - 1) / CONV_BY;
+  const int nbricks = nbx * nby * n1;
+  auto stage = [&](int br, int buf) {
+    const int x0 = br % nbx * CONV_BX, y0 = br / nbx % nby * CONV_BY, z0 = br / (nbx * nby);
+    const unsigned base = sm + buf * WG_STAGE;
+    for (int t = tid; t < WG_HALO * 4; t += 32 * WG_WARPS) {
+      const int node = t >> 2, ch = t & 3;
+      const int gx = x0 - 1 + node % CONV_HX, gy = y0 - 1 + node / CONV_HX % CONV_HY,
+                gz = z0 - 1 + node / (CONV_HX * CONV_HY);
+      const bool on = gx >= 0 && gy >= 0 && gz >= 0 && gx < n1 && gy < n1 && gz < n1;
+      const size_t L = on ? (size_t)gx + (size_t)n1 * ((size_t)gy + (size_t)n1 * gz) : 0;
+      cp_async16(base + swz(node, ch), x + L * 32 + ch * 8, on);
+    }
+    for (int t = tid; t < 3 * WG_NODES * 4; t += 32 * WG_WARPS) {
+      const int node = t >> 2, ch = t & 3, p = node / WG_NODES, i = node % WG_NODES;
+      const int gx = x0 + i % CONV_BX, gy = y0 + i / CONV_BX;
+      const bool on = gx < n1 && gy < n1;
+      const size_t L = on ? (size_t)gx + (size_t)n1 * ((size_t)gy + (size_t)n1 * z0) : 0;
+      cp_async16(base + WG_HALO * 64 + swz(node, ch), dz + ((size_t)p * NL + L) * 32 + ch * 8, on);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  float acc[3][4][4];
+  float *own = reinterpret_cast<float *>(conv_sm + 2 * WG_STAGE) + tid;  // [48][threads]
+#pragma unroll
+  for (int o = 0; o < 3; o++)
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        acc[o][nt][e] = 0.0f;
+        own[((o * 4 + nt) * 4 + e) * 32 * WG_WARPS] = 0.0f;
+      }
+  // lanes of ldmatrix.x4.trans: A tiles (nodes 0-7 | 8-15) x (co 0-7 | 8-15), the
+  // node half in the tile index's high bit; B tiles the other way round
+  const int ti = lane >> 3, tr = lane & 7;
+  const int a_node = (ti >> 1) * 8 + tr, a_ch = 2 * mt + (ti & 1);
+  const int b_node = (ti & 1) * 8 + tr, b_ch = ti >> 1;
+  if (blockIdx.x < nbricks) stage(blockIdx.x, 0);
+  int buf = 0;
+  for (int br = blockIdx.x; br < nbricks; br += gridDim.x, buf ^= 1) {
+    const int next = br + gridDim.x;
+    if (next < nbricks) {
+      stage(next, buf ^ 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    const unsigned s_x = sm + buf * WG_STAGE, s_d = s_x + WG_HALO * 64;
+#pragma unroll 1
+    for (int ks = 0; ks < WG_NODES / 16; ks++) {
+      unsigned a[3][4];
+#pragma unroll
+      for (int p = 0; p < 3; p++) ldsm_x4_t(s_d + swz(p * WG_NODES + ks * 16 + a_node, a_ch), a[p]);
+#pragma unroll
+      for (int o = 0; o < 3; o++) {
+        const int k = 3 * wo + o, dx = k % 3, dy = k / 3 % 3, dzz = k / 9;
+        const int row = b_node + dx + CONV_HX * (ks + dy + CONV_HY * dzz);
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          unsigned b[4];
+          ldsm_x4_t(s_x + swz(row, 2 * p + b_ch), b);
+#pragma unroll
+          for (int q = 2; q >= 0; q--) {
+            mma_bf16(acc[o][2 * p], a[q], b[0], b[1]);
+            mma_bf16(acc[o][2 * p + 1], a[q], b[2], b[3]);
+          }
+        }
+      }
+      if (ks % WG_FLUSH != WG_FLUSH - 1) continue;
+#pragma unroll
+      for (int o = 0; o < 3; o++)
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            own[((o * 4 + nt) * 4 + e) * 32 * WG_WARPS] += acc[o][nt][e];
+            acc[o][nt][e] = 0.0f;
+          }
+    }
+    __syncthreads();  // this brick's reads are done before its buffer is filled again
+  }
+  const int g = lane >> 2, q = lane & 3;
+  float *out = part + (size_t)blockIdx.x * 27 * 1024;
+#pragma unroll
+  for (int o = 0; o < 3; o++)
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        out[((3 * wo + o) * 32 + mt * 16 + g + 8 * (e >> 1)) * 32 + nt * 8 + 2 * q + (e & 1)] =
+            own[((o * 4 + nt) * 4 + e) * 32 * WG_WARPS];
+}
+
+// gw[co][ci][k] += sum over the CTAs' partials; gb[co] likewise.  A block takes 64
+// values, each in four runs of consecutive CTAs (more loads in flight), added
+// in order.
+__global__ void __launch_bounds__(256) k_wgrad_sum(int cin, int cout, int nw, const float *__restrict__ part, int nb,
+                                                   const float *__restrict__ bsum, float *__restrict__ gw,
+                                                   float *__restrict__ gb) {
+  __shared__ float run[4][64];
+  const int t = blockIdx.x * 64 + (threadIdx.x & 63), q = threadIdx.x >> 6;
+  const bool weight = t < 27 * 1024;
+  const int n = weight ? nw : nb, stride = weight ? 27 * 1024 : 32;
+  const float *src = weight ? part + t : bsum + (t - 27 * 1024);
+  float v = 0.0f;
+  if (weight || t < 27 * 1024 + 32) {
+    const int per = (n + 3) / 4, c1 = min(n, (q + 1) * per);
+#pragma unroll 8
+    for (int c = q * per; c < c1; c++) v += src[(size_t)c * stride];
+  }
+  run[q][threadIdx.x & 63] = v;
+  __syncthreads();
+  if (q > 0) return;
+  v = (run[0][threadIdx.x] + run[1][threadIdx.x]) + (run[2][threadIdx.x] + run[3][threadIdx.x]);
+  if (weight) {
+    const int k = t >> 10, co = t >> 5 & 31, ci = t & 31;
+    if (co < cout && ci < cin) gw[((size_t)co * cin + ci) * 27 + k] += v;
+  } else if (t < 27 * 1024 + cout) {
+    gb[t - 27 * 1024] += v;
+  }
 }
 
 // ------------------------------------------------------------- smoothing step
@@ -349,15 +481,13 @@ template int learned_smooth<float>(cudaStream_t, const Level &, const float *, f
 template int learned_smooth<double>(cudaStream_t, const Level &, const double *, double *, double);
 
 // ------------------------------------------------------------- network driver
-static int conv_smem(int cin, int cout) { return cin * cout * 27 * (int)sizeof(float); }
-
 static int set_conv_attrs() {
   static bool done = false;
   if (done) return PMG_OK;
-  PMG_CUDA(cudaFuncSetAttribute(k_conv_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM));
-  PMG_CUDA(cudaFuncSetAttribute(k_conv_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM));
-  PMG_CUDA(cudaFuncSetAttribute(k_conv_bwd_data<NET_C1, NET_C2>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_smem(NET_C1, NET_C2)));
-  PMG_CUDA(cudaFuncSetAttribute(k_conv_bwd_data<NET_C2, NET_C3>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_smem(NET_C2, NET_C3)));
+  PMG_CUDA(cudaFuncSetAttribute(k_conv_tc<CONV_HIDDEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM));
+  PMG_CUDA(cudaFuncSetAttribute(k_conv_tc<CONV_STENCIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM));
+  PMG_CUDA(cudaFuncSetAttribute(k_conv_tc<CONV_GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM));
+  PMG_CUDA(cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM));
   done = true;
   return PMG_OK;
 }
@@ -368,13 +498,14 @@ static int conv_grid(int n1, int num_sms) {
   return (int)std::min<long>(nb, 2L * num_sms);
 }
 
-// forward pass on one level: features -> W (stencil, L.lw_stencil); with
-// train, the FP32 channel-major layer inputs and pre-activations stay in S
+// forward pass on one level: features -> W (stencil, L.lw_stencil).  With train
+// the layers' inputs stay in S.xa, S.xb, S.xc.
 static int net_forward(cudaStream_t s, int num_sms, Level &L, const __nv_bfloat16 *wb, NetScratch &S, bool train) {
   const int n1 = L.lat_n[0], NL = n1 * n1 * n1;
   PMG_TRY(set_conv_attrs());
-  PMG_TRY(S.alloc(NL, NET_C0, NET_C1, NET_C2, train));
+  PMG_TRY(S.alloc(NL, train));
   __nv_bfloat16 *xa = reinterpret_cast<__nv_bfloat16 *>(S.xa.p), *xb = reinterpret_cast<__nv_bfloat16 *>(S.xb.p);
+  __nv_bfloat16 *xc = train ? reinterpret_cast<__nv_bfloat16 *>(S.xc.p) : xa;
   __nv_bfloat16 *wpk = reinterpret_cast<__nv_bfloat16 *>(S.wpk.p);
   const int WPK = 27 * 32 * 32;
   k_pack_weights<<<WPK / 256, 256, 0, s>>>(NET_C0, NET_C1, wb + NET_OFF_W1, wpk);
@@ -382,22 +513,19 @@ static int net_forward(cudaStream_t s, int num_sms, Level &L, const __nv_bfloat1
   k_pack_weights<<<WPK / 256, 256, 0, s>>>(NET_C2, NET_C3, wb + NET_OFF_W3, wpk + 2 * WPK);
   PMG_CUDA(cudaMemsetAsync(xa, 0, sizeof(__nv_bfloat16) * 32 * (size_t)NL, s));
   PMG_CUDA(cudaMemsetAsync(S.dscale.p, 0, sizeof(float) * (size_t)NL, s));
-  if (train) PMG_CUDA(cudaMemsetAsync(S.feat.p, 0, sizeof(float) * NET_C0 * (size_t)NL, s));
-  k_features<<<(L.N + 255) / 256, 256, 0, s>>>(L.N, L.Na, n1, L.rowptr.p, L.kcol.p, L.A.p, L.dof_ijk.p, xa,
-                                                train ? S.feat.p : nullptr, S.dscale.p);
+  k_features<<<(L.N + 255) / 256, 256, 0, s>>>(L.N, L.Na, n1, L.rowptr.p, L.kcol.p, L.A.p, L.dof_ijk.p, xa, S.dscale.p);
   PMG_TRY(L.lw_stencil.alloc((size_t)27 * NL));
   const int g = conv_grid(n1, num_sms);
-  k_conv_tc<false><<<g, 256, CONV_SMEM, s>>>(n1, NET_C1, xa, wpk, wb + NET_OFF_B1, xb, train ? S.a1.p : nullptr,
-                                              train ? S.z1.p : nullptr, nullptr, nullptr);
-  k_conv_tc<false><<<g, 256, CONV_SMEM, s>>>(n1, NET_C2, xb, wpk + WPK, wb + NET_OFF_B2, xa, train ? S.a2.p : nullptr,
-                                              train ? S.z2.p : nullptr, nullptr, nullptr);
-  k_conv_tc<true><<<g, 256, CONV_SMEM, s>>>(n1, NET_C3, xa, wpk + 2 * WPK, wb + NET_OFF_B3, nullptr, nullptr, nullptr,
-                                             S.dscale.p, L.lw_stencil.p);
+  k_conv_tc<CONV_HIDDEN><<<g, 256, CONV_SMEM, s>>>(n1, NET_C1, xa, wpk, wb + NET_OFF_B1, xb, nullptr, nullptr, nullptr,
+                                                   nullptr);
+  k_conv_tc<CONV_HIDDEN><<<g, 256, CONV_SMEM, s>>>(n1, NET_C2, xb, wpk + WPK, wb + NET_OFF_B2, xc, nullptr, nullptr,
+                                                   nullptr, nullptr);
+  k_conv_tc<CONV_STENCIL><<<g, 256, CONV_SMEM, s>>>(n1, NET_C3, xc, wpk + 2 * WPK, wb + NET_OFF_B3, nullptr, S.dscale.p,
+                                                    L.lw_stencil.p, nullptr, nullptr);
   count_launches(7);
   PMG_CUDA(cudaGetLastError());
   return PMG_OK;
 }
-
 
 int learned_forward(Handle &h, Level &L) {
   if (!h.has_learned || L.lat_n[0] <= 0) {
@@ -463,21 +591,41 @@ __global__ void k_spmv_t(int N, const int *__restrict__ rp, const int *__restric
   y[i] = s;
 }
 
-// dout3[k][L] = -du[L] * r[nb_k(L)] * dscale[L]  (active nodes; du in lattice order)
-__global__ void k_train_dout(int NL, int n1, const float *__restrict__ dul, const float *__restrict__ rl,
-                             const float *__restrict__ dscale, float *__restrict__ dout) {
-  const int L = blockIdx.x * blockDim.x + threadIdx.x;
-  if (L >= NL) return;
-  const float g = -dul[L] * dscale[L];
-  for (int k = 0; k < 27; k++) {
-    const int nb = lat_nb(L, k, n1);
-    dout[(size_t)k * NL + L] = nb >= 0 ? g * rl[nb] : 0.0f;
+// The loss's gradient at the last layer's output, dz[k][L] = -du[L] dscale[L] r[nb_k(L)]
+// times 2 / |r|^2, in three BF16 parts (channels 27..31 are 0), and the blocks'
+// sums per channel (bsum[block][32]); a thread takes 8 channels of a node at a time.
+__global__ void __launch_bounds__(256) k_train_dout(int n1, const float *__restrict__ dul, const float *__restrict__ rl,
+                                                    const float *__restrict__ dscale, const double *__restrict__ r2,
+                                                    __nv_bfloat16 *__restrict__ dz, float *__restrict__ bsum) {
+  __shared__ float sb[64][33];
+  const int NL = n1 * n1 * n1, c8 = threadIdx.x & 3;
+  const float f = (float)(2.0 / (*r2 > 0 ? *r2 : 1.0));
+  float bs[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) bs[e] = 0.0f;
+  for (int L = blockIdx.x * 64 + (threadIdx.x >> 2); L < NL; L += gridDim.x * 64) {
+    const float g = -dul[L] * dscale[L];
+    __align__(16) __nv_bfloat16 p[3][8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const int k = c8 * 8 + e;
+      const int nb = k < 27 ? lat_nb(L, k, n1) : -1;
+      const float v = nb >= 0 ? g * rl[nb] * f : 0.0f;
+      bs[e] += v;
+      split3(v, p[0][e], p[1][e], p[2][e]);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      *reinterpret_cast<uint4 *>(dz + ((size_t)q * NL + L) * 32 + c8 * 8) = *reinterpret_cast<const uint4 *>(p[q]);
   }
-}
-
-__global__ void k_scale_f(size_t n, float *x, const double *__restrict__ s2) {
-  const float f = (float)(2.0 / (*s2 > 0 ? *s2 : 1.0));
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) x[i] *= f;
+#pragma unroll
+  for (int e = 0; e < 8; e++) sb[threadIdx.x >> 2][c8 * 8 + e] = bs[e];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    float v = 0.0f;
+    for (int w = 0; w < 64; w++) v += sb[w][threadIdx.x];
+    bsum[blockIdx.x * 32 + threadIdx.x] = v;
+  }
 }
 
 __global__ void k_adam(int n, float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
@@ -621,41 +769,49 @@ int pmg_learned_train_step(pmg_handle hh, int level, int n_samples, const double
     PMG_CUDA(cudaMemsetAsync(h->lw_v.p, 0, sizeof(float) * NET_NPARAM, s));
   }
   PMG_CUDA(cudaMemsetAsync(h->lw_grad.p, 0, sizeof(float) * NET_NPARAM, s));
-  DBuf<float> rl, dul, dout, d2, d1;
-  DBuf<double> u, v, du, nrm;
-  PMG_TRY(rl.alloc(NL)); PMG_TRY(dul.alloc(NL));
-  PMG_TRY(dout.alloc((size_t)NET_C3 * NL)); PMG_TRY(d2.alloc((size_t)NET_C2 * NL)); PMG_TRY(d1.alloc((size_t)NET_C1 * NL));
-  PMG_TRY(u.alloc(N)); PMG_TRY(v.alloc(N)); PMG_TRY(du.alloc(N)); PMG_TRY(nrm.alloc(2 * n_samples));
-  const int gN = (N + 255) / 256, gL = (NL + 255) / 256, gC = (NL + 127) / 128;
-  float *gw = h->lw_grad.p;
+  const int nw = h->num_sms, nb3 = std::min((NL + 63) / 64, 4 * h->num_sms), ngr = conv_grid(n1, h->num_sms);
+  PMG_TRY(S.alloc_backward(NL, N, nw, std::max(nb3, ngr), n_samples));
+  double *u = S.u.p, *v = S.v.p, *du = S.du.p, *nrm = S.nrm.p;
+  const int gN = (N + 255) / 256, WPK = 27 * 32 * 32;
+  float *gw = h->lw_grad.p, *part = S.part.p, *bsum = S.bsum.p;
   const __nv_bfloat16 *wb = reinterpret_cast<const __nv_bfloat16 *>(h->lw_bf16.p);
+  const __nv_bfloat16 *x0 = reinterpret_cast<const __nv_bfloat16 *>(S.xa.p),
+                      *x1 = reinterpret_cast<const __nv_bfloat16 *>(S.xb.p),
+                      *x2 = reinterpret_cast<const __nv_bfloat16 *>(S.xc.p);
+  __nv_bfloat16 *da = reinterpret_cast<__nv_bfloat16 *>(S.da.p), *db = reinterpret_cast<__nv_bfloat16 *>(S.db.p);
+  __nv_bfloat16 *wt = reinterpret_cast<__nv_bfloat16 *>(S.wpk.p) + 3 * WPK;
+  k_pack_weights_t<<<WPK / 256, 256, 0, s>>>(NET_C2, NET_C3, wb + NET_OFF_W3, wt);
+  k_pack_weights_t<<<WPK / 256, 256, 0, s>>>(NET_C1, NET_C2, wb + NET_OFF_W2, wt + WPK);
+  count_launches(2);
+  const int gs = (WPK + 32 + 63) / 64;
+  auto weights = [&](int cin, int cout, const __nv_bfloat16 *dz, const __nv_bfloat16 *x, int nb, int off_w, int off_b) {
+    k_conv_wgrad<<<nw, 32 * WG_WARPS, WG_SMEM, s>>>(n1, dz, x, part);
+    k_wgrad_sum<<<gs, 256, 0, s>>>(cin, cout, nw, part, nb, bsum, gw + off_w, gw + off_b);
+  };
   for (int smp = 0; smp < n_samples; smp++) {
     const double *e = e_dev + (size_t)smp * N, *r = r_dev + (size_t)smp * N;
-    PMG_CUDA(cudaMemsetAsync(rl.p, 0, sizeof(float) * NL, s));
-    k_lat_gather<<<gN, 256, 0, s>>>(N, L.dof_ijk.p, r, rl.p);
-    k_train_apply<<<gN, 256, 0, s>>>(N, L.Na, n1, L.dof_ijk.p, L.lw_stencil.p, rl.p, e, u.p);
-    PMG_TRY(spmv<double>(s, L, L.A.p, u.p, v.p));
-    PMG_TRY(dot(*h, v.p, v.p, N, nrm.p + 2 * smp));
-    PMG_TRY(dot(*h, r, r, N, nrm.p + 2 * smp + 1));
+    PMG_CUDA(cudaMemsetAsync(S.rl.p, 0, sizeof(float) * NL, s));
+    k_lat_gather<<<gN, 256, 0, s>>>(N, L.dof_ijk.p, r, S.rl.p);
+    k_train_apply<<<gN, 256, 0, s>>>(N, L.Na, n1, L.dof_ijk.p, L.lw_stencil.p, S.rl.p, e, u);
+    PMG_TRY(spmv<double>(s, L, L.A.p, u, v));
+    PMG_TRY(dot(*h, v, v, N, nrm + 2 * smp));
+    PMG_TRY(dot(*h, r, r, N, nrm + 2 * smp + 1));
     // dL/dv = 2 v / |r|^2 ; du = A^T dL/dv ; dL/dc = -du
-    k_spmv_t<<<gN, 256, 0, s>>>(N, L.rowptr.p, L.kcol.p, L.tpos.p, L.A.p, v.p, du.p);
-    PMG_CUDA(cudaMemsetAsync(dul.p, 0, sizeof(float) * NL, s));
-    k_lat_gather<<<gN, 256, 0, s>>>(N, L.dof_ijk.p, du.p, dul.p);
-    k_train_dout<<<gL, 256, 0, s>>>(NL, n1, dul.p, rl.p, S.dscale.p, dout.p);
-    k_scale_f<<<std::min(gL * 27, 148 * 16), 256, 0, s>>>((size_t)NET_C3 * NL, dout.p, nrm.p + 2 * smp + 1);
+    k_spmv_t<<<gN, 256, 0, s>>>(N, L.rowptr.p, L.kcol.p, L.tpos.p, L.A.p, v, du);
+    PMG_CUDA(cudaMemsetAsync(S.dul.p, 0, sizeof(float) * NL, s));
+    k_lat_gather<<<gN, 256, 0, s>>>(N, L.dof_ijk.p, du, S.dul.p);
     // layer 3 (no ReLU), layer 2, layer 1
-    k_conv_bwd_weight<NET_C2, NET_C3><<<NET_C2 * 27, 256, 0, s>>>(n1, dout.p, S.a2.p, gw + NET_OFF_W3, gw + NET_OFF_B3);
-    k_conv_bwd_data<NET_C2, NET_C3><<<gC, 128, conv_smem(NET_C2, NET_C3), s>>>(n1, dout.p, wb + NET_OFF_W3, d2.p);
-    k_relu_bwd<<<std::min(gL * 32, 148 * 16), 256, 0, s>>>((size_t)NET_C2 * NL, S.z2.p, d2.p);
-    k_conv_bwd_weight<NET_C1, NET_C2><<<NET_C1 * 27, 256, 0, s>>>(n1, d2.p, S.a1.p, gw + NET_OFF_W2, gw + NET_OFF_B2);
-    k_conv_bwd_data<NET_C1, NET_C2><<<gC, 128, conv_smem(NET_C1, NET_C2), s>>>(n1, d2.p, wb + NET_OFF_W2, d1.p);
-    k_relu_bwd<<<std::min(gL * 32, 148 * 16), 256, 0, s>>>((size_t)NET_C1 * NL, S.z1.p, d1.p);
-    k_conv_bwd_weight<NET_C0, NET_C1><<<NET_C0 * 27, 256, 0, s>>>(n1, d1.p, S.feat.p, gw + NET_OFF_W1, gw + NET_OFF_B1);
-    count_launches(14);
+    k_train_dout<<<nb3, 256, 0, s>>>(n1, S.dul.p, S.rl.p, S.dscale.p, nrm + 2 * smp + 1, da, bsum);
+    weights(NET_C2, NET_C3, da, x2, nb3, NET_OFF_W3, NET_OFF_B3);
+    k_conv_tc<CONV_GRAD><<<ngr, 256, CONV_SMEM, s>>>(n1, 0, da, wt, nullptr, db, nullptr, nullptr, x2, bsum);
+    weights(NET_C1, NET_C2, db, x1, ngr, NET_OFF_W2, NET_OFF_B2);
+    k_conv_tc<CONV_GRAD><<<ngr, 256, CONV_SMEM, s>>>(n1, 0, db, wt + WPK, nullptr, da, nullptr, nullptr, x1, bsum);
+    weights(NET_C0, NET_C1, da, x0, ngr, NET_OFF_W1, NET_OFF_B1);
+    count_launches(13);
     PMG_CUDA(cudaGetLastError());
   }
   std::vector<double> nr(2 * n_samples);
-  PMG_CUDA(cudaMemcpyAsync(nr.data(), nrm.p, sizeof(double) * nr.size(), cudaMemcpyDeviceToHost, s));
+  PMG_CUDA(cudaMemcpyAsync(nr.data(), nrm, sizeof(double) * nr.size(), cudaMemcpyDeviceToHost, s));
   PMG_CUDA(cudaStreamSynchronize(s));
   double loss = 0;
   for (int smp = 0; smp < n_samples; smp++) loss += nr[2 * smp] / (nr[2 * smp + 1] > 0 ? nr[2 * smp + 1] : 1.0);

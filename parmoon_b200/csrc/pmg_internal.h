@@ -191,28 +191,33 @@ struct Level {
   DBuf<double> sell_val64, sell_invd64;
 };
 
-// Activations of the stencil network.  The tensor-core forward reads and
-// writes node-major BF16 (32 channels = 64 bytes per lattice node, two
-// ping-pong buffers); training also keeps FP32 channel-major copies of every
-// layer's input (the BF16-rounded values) and pre-activations for the
-// backward kernels.
+// Activations and gradients of the stencil network: node-major BF16 (32
+// channels = 64 bytes per lattice node).  The forward uses two ping-pong
+// buffers; training keeps every layer's input (xa, xb, xc), and the backward
+// two gradients of three BF16 parts each (da, db) and the CTAs' partial sums.
+// All grow-only: the levels of a hierarchy share the buffers of the largest.
 struct NetScratch {
-  DBuf<uint16_t> xa, xb, wpk;
-  DBuf<float> feat, a1, z1, a2, z2, dscale;
-  // grow-only: the levels of a hierarchy share the buffers of the largest
-  int alloc(int nl, int c0, int c1, int c2, bool train) {
+  DBuf<uint16_t> xa, xb, xc, wpk, da, db;
+  DBuf<float> dscale, rl, dul, part, bsum;
+  DBuf<double> u, v, du, nrm;
+  int alloc(int nl, bool train) {
     PMG_TRY(xa.reserve((size_t)32 * nl));
     PMG_TRY(xb.reserve((size_t)32 * nl));
+    if (train) PMG_TRY(xc.reserve((size_t)32 * nl));
     PMG_TRY(dscale.reserve(nl));
-    PMG_TRY(wpk.reserve((size_t)3 * 27 * 32 * 32));
-    if (train) {
-      PMG_TRY(feat.reserve((size_t)c0 * nl));
-      PMG_TRY(a1.reserve((size_t)c1 * nl));
-      PMG_TRY(z1.reserve((size_t)c1 * nl));
-      PMG_TRY(a2.reserve((size_t)c2 * nl));
-      PMG_TRY(z2.reserve((size_t)c2 * nl));
-    }
-    return PMG_OK;
+    return wpk.reserve((size_t)5 * 27 * 32 * 32);
+  }
+  int alloc_backward(int nl, int n, int n_part, int n_bsum, int n_samples) {
+    PMG_TRY(da.reserve((size_t)96 * nl));
+    PMG_TRY(db.reserve((size_t)96 * nl));
+    PMG_TRY(rl.reserve(nl));
+    PMG_TRY(dul.reserve(nl));
+    PMG_TRY(part.reserve((size_t)n_part * 27 * 32 * 32));
+    PMG_TRY(bsum.reserve((size_t)n_bsum * 32));
+    PMG_TRY(u.reserve(n));
+    PMG_TRY(v.reserve(n));
+    PMG_TRY(du.reserve(n));
+    return nrm.reserve((size_t)2 * n_samples);
   }
 };
 
