@@ -22,8 +22,8 @@
 
 namespace pmg {
 
-constexpr int kNoallocRowsPerBlock = 256;
-constexpr size_t kNoallocPartials = (size_t)PMG_NOALLOC_MAX_ROWS / kNoallocRowsPerBlock;  // 65,536 doubles
+constexpr int kNoallocMostRowsPerBlock = 256;
+constexpr size_t kNoallocPartials = (size_t)PMG_NOALLOC_MAX_ROWS / kNoallocMostRowsPerBlock;  // 65,536 doubles
 
 static __device__ __align__(256) double g_noalloc_partials[kNoallocPartials];
 
@@ -52,27 +52,47 @@ static int noalloc_scratch(int device, double **out) {
   return PMG_OK;
 }
 
-// Block b owns rows [256 b, 256 b + 256): W lanes per row, the block's sum of
+// Block b owns the R rows from R b on: W lanes per row, the block's sum of
 // squared defects goes to partials[b].  Loops are warp-uniform (shuffles).
+// HBM bound (12 bytes per entry) once enough rows are under way: R is the
+// smallest of 32, 64, 128, 256 whose blocks the scratch array has room for.  With
+// 256 rows per block a 69 k-row Q2 level ran on 270 blocks, each group through 32
+// rows one after the other: 47.7 us against 16.2 us.
 template <int W>
-__global__ void __launch_bounds__(256) k_defect_partials(int N, const int *__restrict__ rp, const int *__restrict__ kc,
-                                                         const double *__restrict__ a, const double *__restrict__ x,
-                                                         const double *__restrict__ f, double *__restrict__ d,
-                                                         double *__restrict__ partials) {
-  constexpr int GROUPS = 256 / W;
+__global__ void __launch_bounds__(256) k_defect_partials(int N, int R, const int *__restrict__ rp,
+                                                         const int *__restrict__ kc, const double *__restrict__ a,
+                                                         const double *__restrict__ x, const double *__restrict__ f,
+                                                         double *__restrict__ d, double *__restrict__ partials) {
+  constexpr int GROUPS = 256 / W, U = 4;
   __shared__ double sh[GROUPS];
   const int g = threadIdx.x / W, lane = threadIdx.x & (W - 1);
-  const int row0 = blockIdx.x * kNoallocRowsPerBlock;
+  const int row0 = blockIdx.x * R;
   double acc = 0.0;
-  for (int rr = g; rr < kNoallocRowsPerBlock; rr += GROUPS) {
+  for (int rr = g; rr < R; rr += GROUPS) {
     const int row = row0 + rr;
-    double s = 0.0;
-    if (row < N)
-      for (int k = __ldg(rp + row) + lane; k < __ldg(rp + row + 1); k += W) s += __ldg(a + k) * __ldg(x + __ldg(kc + k));
+    double s = 0.0, fr = 0.0;
+    if (row < N) {
+      const int end = __ldg(rp + row + 1);
+      int k = __ldg(rp + row) + lane;
+      if (lane == 0) fr = __ldg(f + row);
+      // the entries of U steps first, then their x: two round trips for U steps
+      for (; k + (U - 1) * W < end; k += U * W) {
+        double v[U];
+        int c[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          c[u] = __ldg(kc + k + u * W);
+          v[u] = __ldcs(a + k + u * W);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) s += v[u] * __ldg(x + c[u]);
+      }
+      for (; k < end; k += W) s += __ldcs(a + k) * __ldg(x + __ldg(kc + k));
+    }
 #pragma unroll
     for (int o = W / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, W);
     if (lane == 0 && row < N) {
-      const double v = __ldg(f + row) - s;
+      const double v = fr - s;
       d[row] = v;
       acc += v * v;
     }
@@ -87,13 +107,14 @@ __global__ void __launch_bounds__(256) k_defect_partials(int N, const int *__res
 }
 
 // One block adds the nb partials in a fixed order and writes the norm.
-__global__ void __launch_bounds__(256) k_noalloc_norm(int nb, const double *__restrict__ partials, double *norm) {
-  __shared__ double sh[256];
+__global__ void __launch_bounds__(1024) k_noalloc_norm(int nb, const double *__restrict__ partials, double *norm) {
+  __shared__ double sh[1024];
   double t = 0.0;
-  for (int k = threadIdx.x; k < nb; k += 256) t += partials[k];
+#pragma unroll 4
+  for (int k = threadIdx.x; k < nb; k += 1024) t += partials[k];
   sh[threadIdx.x] = t;
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
+  for (int s = 512; s > 0; s >>= 1) {
     if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
     __syncthreads();
   }
@@ -125,12 +146,15 @@ extern "C" int pmg_defect_noalloc(pmg_handle hh, int level, const double *x, con
   double *scratch = nullptr;
   int rc = noalloc_scratch(h->device, &scratch);
   if (rc == PMG_OK) {
-    const int nb = (L.N + kNoallocRowsPerBlock - 1) / kNoallocRowsPerBlock;
+    int R = 32;
+    while (R < kNoallocMostRowsPerBlock && (size_t)(L.N + R - 1) / R > kNoallocPartials) R *= 2;
+    const int nb = (L.N + R - 1) / R;
     const int W = L.avg_row >= 48 ? 32 : (L.avg_row >= 16 ? 16 : 8);
-    if (W == 32) k_defect_partials<32><<<nb, 256, 0, h->stream>>>(L.N, L.rowptr.p, L.kcol.p, L.A.p, x, b, r, scratch);
-    else if (W == 16) k_defect_partials<16><<<nb, 256, 0, h->stream>>>(L.N, L.rowptr.p, L.kcol.p, L.A.p, x, b, r, scratch);
-    else k_defect_partials<8><<<nb, 256, 0, h->stream>>>(L.N, L.rowptr.p, L.kcol.p, L.A.p, x, b, r, scratch);
-    k_noalloc_norm<<<1, 256, 0, h->stream>>>(nb, scratch, norm);
+    const int *rp = L.rowptr.p, *kc = L.kcol.p;
+    if (W == 32) k_defect_partials<32><<<nb, 256, 0, h->stream>>>(L.N, R, rp, kc, L.A.p, x, b, r, scratch);
+    else if (W == 16) k_defect_partials<16><<<nb, 256, 0, h->stream>>>(L.N, R, rp, kc, L.A.p, x, b, r, scratch);
+    else k_defect_partials<8><<<nb, 256, 0, h->stream>>>(L.N, R, rp, kc, L.A.p, x, b, r, scratch);
+    k_noalloc_norm<<<1, 1024, 0, h->stream>>>(nb, scratch, norm);
     count_launches(2);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
