@@ -236,8 +236,8 @@ struct Handle {
   int device = 0;
   int num_sms = 148;
   // coarsest-level dense inverse (FP64)
-  DBuf<double> coarse_lu, coarse_inv, coarse_t;  // active block: LU, inverse; reduced rhs
-  DBuf<int> coarse_piv, coarse_perm;
+  DBuf<double> coarse_lu, coarse_w, coarse_inv, coarse_t;  // active block: work array, pivot rows, inverse; reduced rhs
+  DBuf<int> coarse_piv, coarse_perm;  // pivot row of each column, column of each row
   DBuf<int> coarse_cptr;  // colour pointers of the coarsest level's rows (iterative coarse solve)
   bool coarse_ready = false;
   // FGMRES workspace
@@ -274,6 +274,7 @@ struct Handle {
   DBuf<uint16_t> lw_bf16;
   DBuf<float> lw_master, lw_grad, lw_m, lw_v;
   bool has_learned = false;
+  DBuf<int> setup_scratch;  // set-up of the solve copies (build_sell)
   long adam_t = 0;
   NetScratch net_scratch;
   // learned-smoother guard: V-cycle graph with SSOR, active choice

@@ -2,9 +2,9 @@
 //
 //   vcycle          TMultiGrid3D::Cycle (src/FE/MultiGrid3D.C:449-695) with
 //                   step-length control off; FP64 or FP32 storage/compute
-//   coarse solve    SolveExact (src/FE/MGLevel3D.C:865-906): dense LU with
-//                   partial pivoting of the coarsest matrix, turned into an
-//                   explicit inverse so each V-cycle applies one dense GEMV
+//   coarse solve    SolveExact (src/FE/MGLevel3D.C:865-906): the explicit inverse
+//                   of the coarsest matrix (Gauss-Jordan with partial pivoting),
+//                   so each V-cycle applies one dense GEMV
 //   preconditioner  TMultiGridScaIte::Iterate (src/FE/MultiGridScaIte.C:89-130)
 //   fgmres          TFgmresIte::Iterate, flexible branch (src/FE/FgmresIte.C:245-624):
 //                   right preconditioning, modified Gram-Schmidt, Givens rotations.
@@ -23,220 +23,135 @@ namespace pmg {
 
 int level_invdiag(cudaStream_t s, Level &L, int *flags);
 
-// ----------------------------------------------------------------- coarse LU
-// Blocked right-looking LU with partial pivoting (panel width LU_NB), row-major
-// n x n in global memory:
-//   k_lu_panel   one block factors the (n-k0) x nb panel held in shared memory
-//   k_lu_swap    applies the panel's row interchanges to the other columns
-//   k_lu_trsm    U12 = L11^{-1} A12 (one thread per column)
-//   k_lu_gemm    A22 -= L21 U12 (32 x 32 output tiles)
-// then the inverse is formed in one launch (k_lu_inverse_slab, below).
-constexpr int LU_NB = 32;
-constexpr int LU_MAX_N = 832;  // panel (n x 33 doubles) must fit in 227 KB of shared memory
+// ----------------------------------------------------------------- coarse inverse
+// Inverse of the coarsest level's active block (row-major n x n) by Gauss-Jordan
+// exchange steps with partial pivoting, GJ_NB columns at a time.  An exchange
+// step with pivot (p, j) swaps the roles of unknown j and row p; after all of
+// them, row p_j of the array holds unknown j and column k the old row p_k, so
+// Inv[j][p_k] = M[p_j][k].  Rows stay where they are.
+//   k_gj_panel   one CTA, one thread per row with the panel's entries of the row
+//                in registers: the steps on the panel's own columns; leaves the
+//                new panel in M and the old pivot rows in W
+//   k_gj_update  the other columns, for all rows at once: M_i := (0 for a pivot
+//                row, M_i otherwise) + panel_i W
+//   k_gj_finish  the permutation
+// n / 24 panels of two launches replace an LU (panels in shared memory, row
+// swaps, triangular solves, updates) and a substitution pass for the inverse:
+// n = 729 1.5 ms against 3.5 ms before (23 panels of 60 us, inverse 1.26 ms).  A step
+// is bound by its two CTA barriers, the pivot's reduction and one division (1.7
+// us; a rolled loop, and a search beside the update, were no faster).
+constexpr int GJ_NB = 24, GJ_MAX_N = 832;  // one thread per row: 26 warps, 78 registers
 
-__global__ void __launch_bounds__(1024) k_lu_panel(int n, int k0, int nb, double *A, int *piv, int *flags) {
-  extern __shared__ double S[];  // m x nb, row-major with stride nb + 1 (column reads hit distinct banks)
-  __shared__ double sval[32];
-  __shared__ int sidx[32];
-  __shared__ int spiv;
-  const int m = n - k0, tid = threadIdx.x, nt = blockDim.x, ld = nb + 1;
-  for (int t = tid; t < m * nb; t += nt) S[(t / nb) * ld + t % nb] = A[(size_t)(k0 + t / nb) * n + k0 + t % nb];
-  __syncthreads();
-  for (int j = 0; j < nb; j++) {
-    double best = -1.0;
-    int bi = j;
-    for (int i = j + tid; i < m; i += nt) {
-      double v = fabs(S[i * ld + j]);
-      if (v > best) { best = v; bi = i; }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      double ov = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if ((tid & 31) == 0) { sval[tid >> 5] = best; sidx[tid >> 5] = bi; }
-    __syncthreads();
-    if (tid < 32) {
-      double b = tid < (nt >> 5) ? sval[tid] : -1.0;
-      int p = tid < (nt >> 5) ? sidx[tid] : j;
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, b, o);
-        const int op = __shfl_xor_sync(0xffffffffu, p, o);
-        if (ob > b || (ob == b && op < p)) { b = ob; p = op; }
+__global__ void __launch_bounds__(GJ_MAX_N, 1) k_gj_panel(int n, int k0, double *__restrict__ M, double *__restrict__ W,
+                                                          int *__restrict__ piv, int *__restrict__ col_of, int *flags) {
+  __shared__ unsigned wkey[32];
+  __shared__ int widx[32], chosen[GJ_NB];
+  __shared__ __align__(16) double prow[2][GJ_NB];
+  const int r = threadIdx.x, lane = r & 31, w = r >> 5, nw = blockDim.x >> 5;
+  const int nb = min(GJ_NB, n - k0);
+  pdl_wait();
+  pdl_trigger();
+  double a[GJ_NB];
+#pragma unroll
+  for (int k = 0; k < GJ_NB; k++) a[k] = r < n && k < nb ? M[(size_t)r * n + k0 + k] : 0.0;
+  bool free_row = r < n && (k0 == 0 || col_of[r] < 0);
+  int mine = -1;
+#pragma unroll
+  for (int j = 0; j < GJ_NB; j++) {
+    if (j < nb) {
+      // the free row with the largest |a_j| (compared by the upper half of the double; lowest row on ties)
+      const double v = fabs(a[j]);
+      const unsigned key = free_row && v > 0.0 ? (unsigned)__double2hiint(v) + 1u : 0u;
+      const unsigned top = __reduce_max_sync(0xffffffffu, key);
+      const int first = __ffs(__ballot_sync(0xffffffffu, key == top && free_row)) - 1;
+      if (lane == (first < 0 ? 0 : first)) {
+        wkey[w] = first < 0 ? 0u : top;
+        widx[w] = first < 0 ? -1 : r;
       }
-      if (tid == 0) {
-        spiv = p;
-        piv[k0 + j] = k0 + p;
-        if (!(b > 0.0)) atomicOr(flags, 16);
+      __syncthreads();
+      const int ci = lane < nw ? widx[lane] : -1;
+      const unsigned ck = lane < nw ? wkey[lane] : 0u;
+      const unsigned best = __reduce_max_sync(0xffffffffu, ck);
+      const int from = __ffs(__ballot_sync(0xffffffffu, ck == best && ci >= 0)) - 1;
+      const int p = __shfl_sync(0xffffffffu, ci, from < 0 ? 0 : from);
+      double *pr = prow[j & 1];
+      if (r == p) {
+        if (best == 0u) atomicOr(flags, 16);
+        const double inv = a[j] != 0.0 ? 1.0 / a[j] : 0.0;
+#pragma unroll
+        for (int k = 0; k < GJ_NB; k++) {
+          a[k] = k == j ? inv : a[k] * inv;
+          pr[k] = a[k];
+        }
+        free_row = false;
+        mine = k0 + j;
+        chosen[j] = r;
       }
-    }
-    __syncthreads();
-    const int p = spiv;
-    if (p != j && tid < nb) {
-      double t = S[j * ld + tid];
-      S[j * ld + tid] = S[p * ld + tid];
-      S[p * ld + tid] = t;
-    }
-    __syncthreads();
-    const double d = S[j * ld + j];
-    const double inv = d != 0.0 ? 1.0 / d : 0.0;
-    for (int i = j + 1 + tid; i < m; i += nt) S[i * ld + j] *= inv;
-    __syncthreads();
-    // rank-1 update of the panel: lane = column to the right, warp = row group
-    const int w = nb - j - 1, cc = tid & 31, rg = tid >> 5, ng = nt >> 5;
-    if (cc < w) {
-      const double u = S[j * ld + j + 1 + cc];
-      for (int i = j + 1 + rg; i < m; i += ng) S[i * ld + j + 1 + cc] -= S[i * ld + j] * u;
-    }
-    __syncthreads();
-  }
-  for (int t = tid; t < m * nb; t += nt) A[(size_t)(k0 + t / nb) * n + k0 + t % nb] = S[(t / nb) * ld + t % nb];
-}
-
-// row interchanges of panel k0 on the columns outside the panel
-__global__ void k_lu_swap(int n, int k0, int nb, double *A, const int *__restrict__ piv) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n || (c >= k0 && c < k0 + nb)) return;
-  for (int j = 0; j < nb; j++) {
-    const int p = piv[k0 + j];
-    if (p != k0 + j) {
-      double t = A[(size_t)(k0 + j) * n + c];
-      A[(size_t)(k0 + j) * n + c] = A[(size_t)p * n + c];
-      A[(size_t)p * n + c] = t;
+      __syncthreads();
+      if (r != p) {
+        const double f = a[j];
+        a[j] = 0.0;
+#pragma unroll
+        for (int k = 0; k < GJ_NB; k += 2) {
+          const double2 q = *reinterpret_cast<const double2 *>(pr + k);
+          a[k] -= f * q.x;
+          a[k + 1] -= f * q.y;
+        }
+      }
     }
   }
-}
-
-// U12 = L11^{-1} A12 for the columns right of the panel
-__global__ void k_lu_trsm(int n, int k0, int nb, double *A) {
-  __shared__ double L11[LU_NB][LU_NB];
-  for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) L11[t / nb][t % nb] = A[(size_t)(k0 + t / nb) * n + k0 + t % nb];
+  // the old pivot rows, then the new panel
+  if (r < n)
+#pragma unroll 4
+    for (int q = 0; q < nb; q++) W[(size_t)q * n + r] = M[(size_t)chosen[q] * n + r];
   __syncthreads();
-  const int c = k0 + nb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  double y[LU_NB];
+  if (r < n) {
 #pragma unroll
-  for (int i = 0; i < LU_NB; i++) y[i] = i < nb ? A[(size_t)(k0 + i) * n + c] : 0.0;
-#pragma unroll
-  for (int i = 1; i < LU_NB; i++)
-#pragma unroll
-    for (int j = 0; j < LU_NB; j++)
-      if (j < i && i < nb) y[i] -= L11[i][j] * y[j];
-#pragma unroll
-  for (int i = 0; i < LU_NB; i++)
-    if (i < nb) A[(size_t)(k0 + i) * n + c] = y[i];
+    for (int k = 0; k < GJ_NB; k++)
+      if (k < nb) M[(size_t)r * n + k0 + k] = a[k];
+    if (mine >= 0) {
+      col_of[r] = mine;
+      piv[mine] = r;
+    } else if (k0 == 0) {
+      col_of[r] = -1;
+    }
+  }
 }
 
-// A22 -= L21 U12 on 32 x 32 tiles (k0+nb <= row, col < n)
-__global__ void __launch_bounds__(256) k_lu_gemm(int n, int k0, int nb, double *A) {
-  __shared__ double Ls[32][LU_NB + 1], Us[LU_NB][33];
-  const int r0 = k0 + nb + blockIdx.y * 32, c0 = k0 + nb + blockIdx.x * 32;
-  for (int t = threadIdx.x; t < 32 * LU_NB; t += blockDim.x) {
-    const int a = t / LU_NB, b = t % LU_NB;
-    Ls[a][b] = (r0 + a < n && b < nb) ? A[(size_t)(r0 + a) * n + k0 + b] : 0.0;
+// 32 x 32 tiles of the other columns
+__global__ void __launch_bounds__(256) k_gj_update(int n, int k0, double *__restrict__ M, const double *__restrict__ W,
+                                                   const int *__restrict__ col_of) {
+  __shared__ double Ps[32][GJ_NB + 1], Ws[GJ_NB][33];
+  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32, nb = min(GJ_NB, n - k0);
+  pdl_wait();
+  pdl_trigger();
+  for (int t = threadIdx.x; t < 32 * GJ_NB; t += 256) {
+    const int i = t / GJ_NB, k = t % GJ_NB;
+    Ps[i][k] = r0 + i < n && k < nb ? M[(size_t)(r0 + i) * n + k0 + k] : 0.0;
     const int u = t / 32, v = t % 32;
-    Us[u][v] = (u < nb && c0 + v < n) ? A[(size_t)(k0 + u) * n + c0 + v] : 0.0;
+    Ws[u][v] = u < nb && c0 + v < n ? W[(size_t)u * n + c0 + v] : 0.0;
   }
   __syncthreads();
-  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;  // 8 rows per pass
-  for (int a = ty; a < 32; a += 8) {
-    const int r = r0 + a, c = c0 + tx;
-    if (r >= n || c >= n) continue;
-    double s = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < LU_NB; k++) s += Ls[a][k] * Us[k][tx];
-    A[(size_t)r * n + c] -= s;
+  const int c = c0 + (threadIdx.x & 31);
+  if (c >= n || (c >= k0 && c < k0 + nb)) return;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int i = (threadIdx.x >> 5) + 8 * q, r = r0 + i;
+    if (r >= n) break;
+    const int cj = __ldg(col_of + r);
+    double s = cj >= k0 && cj < k0 + nb ? 0.0 : M[(size_t)r * n + c];
+#pragma unroll
+    for (int k = 0; k < GJ_NB; k++) s += Ps[i][k] * Ws[k][threadIdx.x & 31];
+    M[(size_t)r * n + c] = s;
   }
 }
 
-// Inverse from the factors, X = U^{-1} L^{-1} P: block b of the grid owns
-// the 32 columns [32 b, 32 b + 32) of X and keeps that n x 32 slab in shared
-// memory through both substitutions (left-looking: row i of the slab is
-// finished from the rows already final, L / U streamed from L2), so the whole
-// inverse is one launch; lane = column, warps take rows.
-__global__ void k_lu_perm_identity(int n, const int *__restrict__ piv, int *perm) {
-  // perm[i] = original row that the interchanges bring to position i
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    for (int i = 0; i < n; i++) perm[i] = i;
-    for (int k = 0; k < n; k++) {
-      const int p = piv[k];
-      if (p != k) { int t = perm[k]; perm[k] = perm[p]; perm[p] = t; }
-    }
-  }
-}
-
-constexpr int INV_COLS = 16, INV_THREADS = 256, INV_ROWS = INV_THREADS / INV_COLS;
-__global__ void __launch_bounds__(INV_THREADS) k_lu_inverse_slab(int n, const double *__restrict__ LU,
-                                                                const int *__restrict__ perm, double *Inv) {
-  extern __shared__ double sm[];
-  double *Xs = sm;           // n x INV_COLS, the block's columns of X
-  double *Rb = sm + (size_t)n * INV_COLS;  // INV_ROWS rows of L or U, staged
-  const int tid = threadIdx.x, rr = tid / INV_COLS, col = tid % INV_COLS;
-  const int warp = tid >> 5, lane = tid & 31, nwarps = INV_THREADS / 32;
-  const int c = blockIdx.x * INV_COLS + col;
-  for (int i = rr; i < n; i += INV_ROWS) Xs[i * INV_COLS + col] = (c < n && __ldg(perm + i) == c) ? 1.0 : 0.0;
-  // forward with the unit lower factor, INV_ROWS rows per group
-  for (int i0 = 0; i0 < n; i0 += INV_ROWS) {
-    const int rows = min(INV_ROWS, n - i0), width = i0 + rows;
-    __syncthreads();
-    for (int r = warp; r < rows; r += nwarps)
-      for (int k = lane; k < width; k += 32) Rb[r * width + k] = __ldg(LU + (size_t)(i0 + r) * n + k);
-    __syncthreads();
-    double s = 0.0;
-    if (rr < rows) {
-      const double *Lr = Rb + rr * width;
-      double s1 = 0.0;
-      int k = 0;
-      for (; k + 2 <= i0; k += 2) {
-        s += Lr[k] * Xs[k * INV_COLS + col];
-        s1 += Lr[k + 1] * Xs[(k + 1) * INV_COLS + col];
-      }
-      if (k < i0) s += Lr[k] * Xs[k * INV_COLS + col];
-      s += s1;
-    }
-    for (int r = 0; r < rows; r++) {
-      if (rr == r) {
-        const double *Lr = Rb + r * width;
-        double t = Xs[(i0 + r) * INV_COLS + col] - s;
-        for (int k = i0; k < i0 + r; k++) t -= Lr[k] * Xs[k * INV_COLS + col];
-        Xs[(i0 + r) * INV_COLS + col] = t;
-      }
-      __syncthreads();
-    }
-  }
-  // backward with the upper factor, from the last rows
-  for (int i1 = n; i1 > 0; i1 -= INV_ROWS) {
-    const int lo = max(0, i1 - INV_ROWS), rows = i1 - lo, width = n - lo;
-    __syncthreads();
-    for (int r = warp; r < rows; r += nwarps)
-      for (int k = lane; k < width; k += 32) Rb[r * width + k] = __ldg(LU + (size_t)(lo + r) * n + lo + k);
-    __syncthreads();
-    const int i = i1 - 1 - rr;  // the row this thread sums for
-    double s = 0.0;
-    if (rr < rows) {
-      const double *Ur = Rb + (i - lo) * width - lo;  // Ur[k] = U[i][k] for k >= lo
-      double s1 = 0.0;
-      int k = i1;
-      for (; k + 2 <= n; k += 2) {
-        s += Ur[k] * Xs[k * INV_COLS + col];
-        s1 += Ur[k + 1] * Xs[(k + 1) * INV_COLS + col];
-      }
-      if (k < n) s += Ur[k] * Xs[k * INV_COLS + col];
-      s += s1;
-    }
-    for (int r = 0; r < rows; r++) {
-      const int row = i1 - 1 - r;
-      if (rr == r) {
-        const double *Ur = Rb + (row - lo) * width - lo;
-        double t = Xs[row * INV_COLS + col] - s;
-        for (int k = row + 1; k < i1; k++) t -= Ur[k] * Xs[k * INV_COLS + col];
-        Xs[row * INV_COLS + col] = t / Ur[row];
-      }
-      __syncthreads();
-    }
-  }
-  if (c < n)
-    for (int i = rr; i < n; i += INV_ROWS) Inv[(size_t)i * n + c] = Xs[i * INV_COLS + col];
+__global__ void k_gj_finish(int n, const double *__restrict__ M, const int *__restrict__ piv, double *__restrict__ Inv) {
+  pdl_wait();
+  pdl_trigger();
+  const int j = blockIdx.x;
+  const double *row = M + (size_t)piv[j] * n;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) Inv[(size_t)j * n + piv[k]] = row[k];
 }
 
 // the coarsest level's rhs reduced to its active rows: t = f_a - A_ad f_d
@@ -294,7 +209,7 @@ static int coarse_factor_launch(Handle &h, cudaStream_t s) {
   // Dirichlet rows are identity rows, so only the active block is factored:
   // x_a = A_aa^{-1} (f_a - A_ad f_d), x_d = f_d
   const int n = L.Na;
-  if (n > LU_MAX_N) {
+  if (n > GJ_MAX_N) {
     set_error("coarsest level has too many active rows for the dense direct solve (> 832); use the SSOR coarse smoother");
     return PMG_ERR_UNSUPPORTED;
   }
@@ -305,35 +220,24 @@ static int coarse_factor_launch(Handle &h, cudaStream_t s) {
   }
   PMG_TRY(h.coarse_lu.alloc((size_t)n * n));
   PMG_TRY(h.coarse_inv.alloc((size_t)n * n));
+  PMG_TRY(h.coarse_w.alloc((size_t)GJ_NB * n));
   PMG_TRY(h.coarse_piv.alloc(n));
-  PMG_CUDA(cudaMemsetAsync(h.coarse_flags.p, 0, sizeof(int) * 4, s));
-  k_csr_to_dense_active<<<n, 256, 0, s>>>(n, L.rowptr.p, L.kcol.p, L.A.p, h.coarse_lu.p); count_launches(1);
-  static bool attr = false;
-  if (!attr) {
-    PMG_CUDA(cudaFuncSetAttribute(k_lu_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, LU_MAX_N * (LU_NB + 1) * 8));
-    PMG_CUDA(cudaFuncSetAttribute(k_lu_inverse_slab, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  LU_MAX_N * 2 * INV_COLS * 8));
-    attr = true;
-  }
-  for (int k0 = 0; k0 < n; k0 += LU_NB) {
-    const int nb = std::min(LU_NB, n - k0);
-    k_lu_panel<<<1, 1024, (size_t)(n - k0) * (nb + 1) * 8, s>>>(n, k0, nb, h.coarse_lu.p, h.coarse_piv.p, h.coarse_flags.p);
-    k_lu_swap<<<(n + 255) / 256, 256, 0, s>>>(n, k0, nb, h.coarse_lu.p, h.coarse_piv.p);
-    count_launches(2);
-    const int rest = n - k0 - nb;
-    if (rest > 0) {
-      k_lu_trsm<<<(rest + 127) / 128, 128, 0, s>>>(n, k0, nb, h.coarse_lu.p);
-      dim3 g((rest + 31) / 32, (rest + 31) / 32);
-      k_lu_gemm<<<g, 256, 0, s>>>(n, k0, nb, h.coarse_lu.p);
-      count_launches(2);
-    }
-  }
   PMG_TRY(h.coarse_perm.alloc(n));
-  k_lu_perm_identity<<<1, 32, 0, s>>>(n, h.coarse_piv.p, h.coarse_perm.p);
-  k_lu_inverse_slab<<<(n + INV_COLS - 1) / INV_COLS, INV_THREADS, (size_t)n * 2 * INV_COLS * 8, s>>>(
-      n, h.coarse_lu.p, h.coarse_perm.p, h.coarse_inv.p);
-  count_launches(2);
+  PMG_CUDA(cudaMemsetAsync(h.coarse_flags.p, 0, sizeof(int) * 4, s));
+  double *M = h.coarse_lu.p;
+  k_csr_to_dense_active<<<n, 256, 0, s>>>(n, L.rowptr.p, L.kcol.p, L.A.p, M);
   PMG_CUDA(cudaGetLastError());
+  const int tiles = (n + 31) / 32;
+  for (int k0 = 0; k0 < n; k0 += GJ_NB) {
+    PMG_CUDA(launch_pdl(k_gj_panel, dim3(1), dim3(tiles * 32), 0, s, n, k0, M, h.coarse_w.p, h.coarse_piv.p,
+                        h.coarse_perm.p, h.coarse_flags.p));
+    PMG_CUDA(launch_pdl(k_gj_update, dim3(tiles, tiles), dim3(256), 0, s, n, k0, M, (const double *)h.coarse_w.p,
+                        (const int *)h.coarse_perm.p));
+    count_launches(2);
+  }
+  PMG_CUDA(launch_pdl(k_gj_finish, dim3(n), dim3(256), 0, s, n, (const double *)M, (const int *)h.coarse_piv.p,
+                      h.coarse_inv.p));
+  count_launches(2);
   PMG_CUDA(cudaMemcpyAsync(h.h_coarse_flags, h.coarse_flags.p, sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
   return PMG_OK;
 }
