@@ -93,12 +93,13 @@ constexpr int BLK_TASK = 16;  // bytes per task kept beside it
 // Phases and blocks of a level: phase boundaries into L.blk_col (empty: none),
 // block of every active row into blk.  About the cube root of the number of
 // colours as the number of phases first (27 -> 3, 8 -> 2), then finer ones.
-static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std::vector<int> &blk) {
+// d_phase, d_parent: N ints of device scratch each.
+static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std::vector<int> &blk, int *d_phase,
+                       int *d_parent) {
   const int N = L.N, Na = L.Na, nc = (int)L.rcolor_ptr.size() - 1;
   L.blk_col.clear();
   if (N < BLK_MIN_ROWS || nc < 3) return PMG_OK;
   const int s0 = std::max(2, (int)(cbrt((double)nc) + 0.5));
-  DBuf<int> dphase, dparent;
   std::vector<int> phase(N), label(Na);
   for (int S : {s0, s0 + 1, s0 * s0}) {
     if (S >= nc) break;
@@ -108,14 +109,13 @@ static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std:
     for (int p = 0; p < S; p++)
       for (int c = bound[p]; c < bound[p + 1]; c++) phase_of[c] = p;
     for (int r = 0; r < N; r++) phase[r] = phase_of[colour[r]];
-    PMG_TRY(dphase.upload(phase.data(), N, h.stream));
-    PMG_TRY(dparent.alloc(Na));
-    k_cc_init<<<(Na + 255) / 256, 256, 0, h.stream>>>(Na, dparent.p);
-    k_cc_unite<<<h.num_sms * 8, 256, 0, h.stream>>>(Na, L.rowptr.p, L.kcol.p, dphase.p, dparent.p);
-    k_cc_flatten<<<(Na + 255) / 256, 256, 0, h.stream>>>(Na, dparent.p);
+    PMG_CUDA(cudaMemcpyAsync(d_phase, phase.data(), sizeof(int) * N, cudaMemcpyHostToDevice, h.stream));
+    k_cc_init<<<(Na + 255) / 256, 256, 0, h.stream>>>(Na, d_parent);
+    k_cc_unite<<<h.num_sms * 8, 256, 0, h.stream>>>(Na, L.rowptr.p, L.kcol.p, d_phase, d_parent);
+    k_cc_flatten<<<(Na + 255) / 256, 256, 0, h.stream>>>(Na, d_parent);
     count_launches(3);
     PMG_CUDA(cudaGetLastError());
-    PMG_CUDA(cudaMemcpyAsync(label.data(), dparent.p, sizeof(int) * Na, cudaMemcpyDeviceToHost, h.stream));
+    PMG_CUDA(cudaMemcpyAsync(label.data(), d_parent, sizeof(int) * Na, cudaMemcpyDeviceToHost, h.stream));
     PMG_CUDA(cudaStreamSynchronize(h.stream));
     // number the blocks of each phase by their first rows; rows per block and colour
     std::vector<int> n(S, 0);
@@ -279,8 +279,15 @@ int build_sell(Handle &h, Level &L) {
   std::vector<int> colour(N, nc);
   for (int g = 0; g < nc; g++)
     for (int k = L.rcolor_ptr[g]; k < L.rcolor_ptr[g + 1]; k++) colour[L.h_row_list[k]] = g;
+  // device scratch of the set-up, in one allocation that stays with the handle
+  // (an allocation can take longer than all the kernels here)
+  // (a slice holds a row, so there are at most N; even parts keep 8-byte alignment)
+  const size_t part = ((size_t)N + nc + 64) / 2 * 2;
+  PMG_TRY(h.setup_scratch.reserve(7 * part));
+  int *d_colour = h.setup_scratch.p, *d_phase = d_colour + part, *d_nlow = d_phase + part, *d_lptr = d_nlow + part,
+      *d_slot = d_lptr + part, *d_rowa = d_slot + part, *d_bad = d_rowa + part;
   std::vector<int> blk;  // block of each active row inside its phase
-  PMG_TRY(find_blocks(h, L, colour, blk));
+  PMG_TRY(find_blocks(h, L, colour, blk, d_rowa, d_nlow));
   std::vector<int> phase(nc + 1, -1);
   for (size_t p = 0; p + 1 < L.blk_col.size(); p++)
     for (int c = L.blk_col[p]; c < L.blk_col[p + 1]; c++) phase[c] = (int)p;
@@ -290,24 +297,24 @@ int build_sell(Handle &h, Level &L) {
   // higher colour and the sweeps read whole rows.
   std::vector<int> alen(N), nlow(N);
   std::vector<unsigned> ins(N);
-  DBuf<int> d_colour, d_phase, d_nlow, d_bad;
-  DBuf<unsigned> d_ins;
+  unsigned *d_ins = reinterpret_cast<unsigned *>(d_rowa);
   int bad = 0;
-  PMG_TRY(d_colour.upload(colour.data(), N, h.stream));
-  PMG_TRY(d_phase.upload(phase.data(), phase.size(), h.stream));
+  auto put = [&](int *d, const std::vector<int> &v) {
+    return v.empty() ? cudaSuccess
+                     : cudaMemcpyAsync(d, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, h.stream);
+  };
+  PMG_CUDA(put(d_colour, colour));
+  PMG_CUDA(put(d_phase, phase));
   PMG_TRY(L.sell_alen.alloc(N));
-  PMG_TRY(d_nlow.alloc(N));
-  PMG_TRY(d_ins.alloc(N));
-  PMG_TRY(d_bad.alloc(1));
-  PMG_CUDA(cudaMemsetAsync(d_bad.p, 0, sizeof(int), h.stream));
-  k_row_counts<<<h.num_sms * 8, 256, 0, h.stream>>>(N, Na, L.rowptr.p, L.kcol.p, d_colour.p, d_phase.p, L.sell_alen.p,
-                                                    d_nlow.p, d_ins.p, d_bad.p);
+  PMG_CUDA(cudaMemsetAsync(d_bad, 0, 8 * sizeof(int), h.stream));
+  k_row_counts<<<h.num_sms * 8, 256, 0, h.stream>>>(N, Na, L.rowptr.p, L.kcol.p, d_colour, d_phase, L.sell_alen.p,
+                                                    d_nlow, d_ins, d_bad);
   count_launches(1);
   PMG_CUDA(cudaGetLastError());
   PMG_CUDA(cudaMemcpyAsync(alen.data(), L.sell_alen.p, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
-  PMG_CUDA(cudaMemcpyAsync(nlow.data(), d_nlow.p, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
-  PMG_CUDA(cudaMemcpyAsync(ins.data(), d_ins.p, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
-  PMG_CUDA(cudaMemcpyAsync(&bad, d_bad.p, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+  PMG_CUDA(cudaMemcpyAsync(nlow.data(), d_nlow, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
+  PMG_CUDA(cudaMemcpyAsync(ins.data(), d_ins, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
+  PMG_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
   PMG_CUDA(cudaStreamSynchronize(h.stream));
   bool split = bad == 0;
   // (the blocks' tables keep the inside counts in 12 bits)
@@ -445,13 +452,10 @@ int build_sell(Handle &h, Level &L) {
   PMG_TRY(L.blk_meta.upload(meta.data(), meta.size(), h.stream));
   PMG_TRY(L.blk_rows.upload(brows.data(), brows.size(), h.stream));
   // the slices' columns, filled on the device
-  DBuf<int> d_lptr, d_slot;
-  DBuf<unsigned long long> d_nnz;
-  unsigned long long nnz[2] = {0, 0};
-  PMG_TRY(d_lptr.upload(lptr.data(), lptr.size(), h.stream));
-  PMG_TRY(d_slot.upload(slot.data(), slot.size(), h.stream));
-  PMG_TRY(d_phase.upload(phase.data(), phase.size(), h.stream));
-  PMG_TRY(d_nnz.upload(nnz, 2, h.stream));
+  unsigned long long *d_nnz = reinterpret_cast<unsigned long long *>(d_bad + 2), nnz[2] = {0, 0};
+  PMG_CUDA(put(d_lptr, lptr));
+  PMG_CUDA(put(d_slot, slot));
+  PMG_CUDA(put(d_phase, phase));
   PMG_TRY(L.sell_col.alloc(total));
   PMG_TRY(L.sell_c16.alloc(total));
   PMG_TRY(L.sell_src.alloc(split ? total : 0));
@@ -459,13 +463,13 @@ int build_sell(Handle &h, Level &L) {
   PMG_TRY(L.sell_loc.alloc((size_t)total_in * 128));
   if (nslices > 0) {
     k_sell_fill<<<std::min((nslices + 7) / 8, h.num_sms * 16), 256, 0, h.stream>>>(
-        nslices, Na, split, L.sell_perm.p, L.sell_ptr.p, L.sell_nlow.p, L.sell_in.p, d_lptr.p, L.rowptr.p, L.kcol.p,
-        L.sell_alen.p, d_colour.p, d_phase.p, d_slot.p, L.sell_col.p, L.sell_c16.p, L.sell_src.p, L.sell_loc.p,
-        L.sell_wide.p, d_nnz.p);
+        nslices, Na, split, L.sell_perm.p, L.sell_ptr.p, L.sell_nlow.p, L.sell_in.p, d_lptr, L.rowptr.p, L.kcol.p,
+        L.sell_alen.p, d_colour, d_phase, d_slot, L.sell_col.p, L.sell_c16.p, L.sell_src.p, L.sell_loc.p,
+        L.sell_wide.p, d_nnz);
     count_launches(1);
     PMG_CUDA(cudaGetLastError());
   }
-  PMG_CUDA(cudaMemcpyAsync(nnz, d_nnz.p, sizeof(nnz), cudaMemcpyDeviceToHost, h.stream));
+  PMG_CUDA(cudaMemcpyAsync(nnz, d_nnz, sizeof(nnz), cudaMemcpyDeviceToHost, h.stream));
   L.n_dd = (int)dd_row.size();
   PMG_TRY(L.dd_row.upload(dd_row.data(), dd_row.size(), h.stream));
   PMG_TRY(L.dd_beg.upload(dd_beg.data(), dd_beg.size(), h.stream));
