@@ -333,6 +333,7 @@ int pmg_set_level_mesh(pmg_handle hh, int level, int elem_type, int n_cells, con
   L.ecolor_ptr = ptr;
   L.cell_order = order;
   L.ctab.release();
+  L.d_cell_order.release();
   L.ctab_nq = 0;
   PMG_TRY(L.elem_dof.upload(ed.data(), ed.size(), h->stream));
   PMG_TRY(L.cell_vert.upload(cv.data(), cv.size(), h->stream));

@@ -127,6 +127,7 @@ struct Level {
   // tabulated coefficients (PMG_COEF_TABLE): n_cells x ctab_nq x 6, colour order
   DBuf<double> ctab;
   int ctab_nq = 0;
+  DBuf<int> d_cell_order;
   // multicolour SSOR row lists (active rows only), grouped by colour
   DBuf<int> row_list;
   std::vector<int> rcolor_ptr;
@@ -274,6 +275,7 @@ struct Handle {
   DBuf<uint16_t> lw_bf16;
   DBuf<float> lw_master, lw_grad, lw_m, lw_v;
   bool has_learned = false;
+  DBuf<double> ctab_in;     // a coefficient table in the caller's cell order
   DBuf<int> setup_scratch;  // set-up of the solve copies (build_sell)
   long adam_t = 0;
   NetScratch net_scratch;
