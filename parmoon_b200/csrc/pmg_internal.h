@@ -247,6 +247,7 @@ struct Handle {
   DBuf<double> red_partial;
   DBuf<double> slc_part;  // step-length control: block partials of (d0, y), (y, y) and alpha
   DBuf<unsigned int> red_counter;
+  DBuf<double> gs_part, gs_rows;  // Gram-Schmidt: block sums; products of the basis vectors
   double *h_H = nullptr;  // pinned mirror of one Hessenberg column
   // error flags written by kernels (slot lookups, non-finite values)
   DBuf<int> d_flags;
@@ -317,6 +318,7 @@ int convert_f64_f32(cudaStream_t s, const double *a, float *b, size_t n);
 int copy_dirichlet(cudaStream_t s, int Na, int N, const double *f, double *x);
 int dot(Handle &h, const double *a, const double *b, size_t n, double *result_dev);
 // w -= (*hk_dev) vk, then *h_next = w . u (u = w: the squared norm)
+int arnoldi_column(Handle &h, size_t n, int i, double *V, double *w, double *hc, double *hc_host);
 int mgs_step(Handle &h, size_t n, const double *hk_dev, const double *vk, const double *u, double *w, double *h_next);
 int scale_by_inv_sqrt(cudaStream_t s, size_t n, const double *nrm2_dev, const double *x, double *y);
 int fill(cudaStream_t s, double *x, double v, size_t n);

@@ -799,12 +799,8 @@ int solve(Handle &h, double *sol_host, const double *rhs_host, pmg_solve_stats *
       PMG_TRY(sell_spmv<double>(s, F, zi, nullptr, w, 0, h.num_sms));
       double *Hc = Hd + (size_t)i * (m + 1);
       // modified Gram-Schmidt (FgmresIte.C): h_k = w.v_k, w -= h_k v_k for
-      // k = 0..i, then h_{i+1}^2 = w.w; each update fused with the next product
-      PMG_TRY(dot(h, w, V, N, Hc));
-      for (int k = 0; k <= i; k++)
-        PMG_TRY(mgs_step(h, N, Hc + k, V + (size_t)k * N, k < i ? V + (size_t)(k + 1) * N : w, w, Hc + k + 1));
-      PMG_TRY(scale_by_inv_sqrt(s, N, Hc + i + 1, w, V + (size_t)(i + 1) * N));
-      PMG_CUDA(cudaMemcpyAsync(hcol, Hc, sizeof(double) * (i + 2), cudaMemcpyDeviceToHost, s));
+      // k = 0..i, then h_{i+1}^2 = w.w and v_{i+1} = w / h_{i+1}
+      PMG_TRY(arnoldi_column(h, N, i, V, w, Hc, hcol));
       PMG_CUDA(cudaStreamSynchronize(s));
       for (int k = 0; k <= i; k++) H[(size_t)k * m + i] = hcol[k];
       H[(size_t)(i + 1) * m + i] = sqrt(hcol[i + 1]);

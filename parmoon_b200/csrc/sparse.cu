@@ -360,6 +360,169 @@ int mgs_step(Handle &h, size_t n, const double *hk_dev, const double *vk, const 
   return PMG_OK;
 }
 
+// A column of modified Gram-Schmidt (h_k = w.v_k, w -= h_k v_k for k = 0..i) with
+// all inner products taken at once (Swirydowicz, Langou, Ananthan, Yang, Thomas,
+// Low synchronization Gram-Schmidt and GMRES algorithms, 2020): with c_k = w.v_k of
+// the w that comes in and l_rk = v_r.v_k (of the order of the rounding, not zero),
+//   h_r = c_r - sum_{k<r} l_rk h_k
+// is what the step-by-step form computes, so w loses the same components in the
+// same order.  The row l_i is taken in the same pass as c.  Three launches per
+// column instead of i + 3, and V passes twice through memory where the steps
+// moved four vectors each (w in and out, v_k, v_{k+1}).  The kernels of the 20
+// columns of the Q2 64^3 solve (2.1 M rows): 5.0 ms -> 2.8 ms, half of it at the
+// HBM rate of V; whole solves 54.1 -> 53.4 ms, Q1 32^3 (36 k rows) 1.96 -> 1.84 ms.
+// (One cooperative launch per column with w on the chip was slower at every size:
+// an exchange of sums between all SMs takes 4.4 us, a launch 3.)
+// The partial sums are added in a fixed order by every block for itself.
+constexpr int GS_THREADS = 512;
+constexpr int GS_K = 8;  // vectors per pass over w: 16 sums in registers, 9 loads in flight
+constexpr int GS_MAX = 61;
+
+__device__ inline double gs_partials(const double *part, int nblk, int lane) {
+  double t = 0;
+  for (int b = lane; b < nblk; b += 32) t += __ldcg(part + b);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+// part[2k] = w.v_k, part[2k + 1] = v_i.v_k (k < i), per block
+__global__ void __launch_bounds__(GS_THREADS, 2) k_gs_dots(size_t n, int i, const double *__restrict__ V,
+                                                           const double *__restrict__ w, double *part) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ double sh[GS_THREADS / 32][2 * GS_K];
+  const size_t st = (size_t)gridDim.x * GS_THREADS;
+  const double *vi = V + (size_t)i * n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int k0 = 0; k0 <= i; k0 += GS_K) {
+    const int kc = min(GS_K, i + 1 - k0);
+    const double *vk = V + (size_t)k0 * n;
+    double c[GS_K], l[GS_K];
+#pragma unroll
+    for (int k = 0; k < GS_K; k++) c[k] = l[k] = 0;
+    for (size_t e = (size_t)blockIdx.x * GS_THREADS + threadIdx.x; e < n; e += st) {
+      double v[GS_K];
+#pragma unroll
+      for (int k = 0; k < GS_K; k++) v[k] = k < kc ? __ldg(vk + (size_t)k * n + e) : 0.0;
+      const double we = __ldg(w + e), ve = __ldg(vi + e);
+#pragma unroll
+      for (int k = 0; k < GS_K; k++) {
+        c[k] += we * v[k];
+        l[k] += ve * v[k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < GS_K; k++) {
+      if (k >= kc) break;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        c[k] += __shfl_xor_sync(0xffffffffu, c[k], o);
+        l[k] += __shfl_xor_sync(0xffffffffu, l[k], o);
+      }
+      if (lane == 0) {
+        sh[warp][2 * k] = c[k];
+        sh[warp][2 * k + 1] = l[k];
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * kc) {
+      double t = 0;
+      for (int q = 0; q < GS_THREADS / 32; q++) t += sh[q][threadIdx.x];
+      part[(size_t)(2 * k0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
+    }
+    __syncthreads();
+  }
+}
+
+// h from the partial sums (every block the same), w -= sum_k h_k v_k in the order
+// of k, and the partial sums of w.w; L: the rows l_r, r < i, of the columns before
+__global__ void __launch_bounds__(GS_THREADS, 2) k_gs_update(size_t n, int i, const double *__restrict__ V, double *w,
+                                                             const double *part, int nblk, double *L, double *h,
+                                                             double *h_host, double *part_w) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ double hs[GS_MAX + 3], li[GS_MAX + 3], sh[GS_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j = warp; j < 2 * i + 1; j += GS_THREADS / 32) {  // (l_ii is not needed)
+    const double t = gs_partials(part + (size_t)j * nblk, nblk, lane);
+    if (lane == 0) (j & 1 ? li : hs)[j >> 1] = t;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    // forward substitution, two rows per lane
+    double c0 = lane <= i ? hs[lane] : 0.0, c1 = lane + 32 <= i ? hs[lane + 32] : 0.0;
+    for (int k = 0; k < i; k++) {
+      const double hk = __shfl_sync(0xffffffffu, k < 32 ? c0 : c1, k & 31);
+      if (lane > k && lane <= i) c0 -= (lane == i ? li[k] : __ldg(L + lane * GS_MAX + k)) * hk;
+      if (lane + 32 > k && lane + 32 <= i)
+        c1 -= (lane + 32 == i ? li[k] : __ldg(L + (lane + 32) * GS_MAX + k)) * hk;
+    }
+    if (lane <= i) hs[lane] = c0;
+    if (lane + 32 <= i) hs[lane + 32] = c1;
+  }
+  __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x <= i) {
+    h[threadIdx.x] = h_host[threadIdx.x] = hs[threadIdx.x];
+    if (threadIdx.x < i) L[i * GS_MAX + threadIdx.x] = li[threadIdx.x];
+  }
+  double s = 0;
+  const size_t st = (size_t)gridDim.x * GS_THREADS;
+  // from the end: what the products read last is still in L2
+  for (size_t r = (size_t)blockIdx.x * GS_THREADS + threadIdx.x; r < n; r += st) {
+    const size_t e = n - 1 - r;
+    double we = w[e];
+    for (int k0 = 0; k0 <= i; k0 += GS_K) {
+      double v[GS_K];
+#pragma unroll
+      for (int k = 0; k < GS_K; k++) v[k] = k0 + k <= i ? __ldg(V + (size_t)(k0 + k) * n + e) : 0.0;
+#pragma unroll
+      for (int k = 0; k < GS_K; k++)
+        if (k0 + k <= i) we -= hs[k0 + k] * v[k];
+    }
+    w[e] = we;
+    s += we * we;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) sh[warp] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0;
+    for (int q = 0; q < GS_THREADS / 32; q++) t += sh[q];
+    part_w[blockIdx.x] = t;
+  }
+}
+
+// h_{i+1}^2 = w.w and v_{i+1} = w / h_{i+1}  (0 -> 0)
+__global__ void __launch_bounds__(GS_THREADS, 2) k_gs_scale(size_t n, const double *__restrict__ w,
+                                                            const double *part_w, int nblk, double *__restrict__ v,
+                                                            double *h, double *h_host) {
+  pdl_wait();
+  pdl_trigger();
+  const double t = gs_partials(part_w, nblk, threadIdx.x & 31);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *h = *h_host = t;
+  const double nv = sqrt(t), sc = nv > 0 ? 1.0 / nv : 0.0;
+  for (size_t e = (size_t)blockIdx.x * GS_THREADS + threadIdx.x; e < n; e += (size_t)gridDim.x * GS_THREADS)
+    v[e] = w[e] * sc;
+}
+
+// Column i of the Arnoldi process: h_0 .. h_i and h_{i+1}^2 to hc and to the pinned
+// hc_host, v_{i+1} to V; w is overwritten.
+int arnoldi_column(Handle &h, size_t n, int i, double *V, double *w, double *hc, double *hc_host) {
+  const int blocks = (int)std::min<size_t>((n + GS_THREADS - 1) / GS_THREADS, (size_t)h.num_sms * 2);
+  PMG_TRY(h.gs_part.reserve((size_t)(2 * GS_MAX + 1) * blocks));
+  PMG_TRY(h.gs_rows.reserve((size_t)GS_MAX * GS_MAX));
+  double *part_w = h.gs_part.p + (size_t)2 * GS_MAX * blocks;
+  PMG_CUDA(launch_pdl(k_gs_dots, dim3(blocks), dim3(GS_THREADS), 0, h.stream, n, i, V, w, h.gs_part.p));
+  PMG_CUDA(launch_pdl(k_gs_update, dim3(blocks), dim3(GS_THREADS), 0, h.stream, n, i, V, w, h.gs_part.p, blocks,
+                      h.gs_rows.p, hc, hc_host, part_w));
+  PMG_CUDA(launch_pdl(k_gs_scale, dim3(blocks), dim3(GS_THREADS), 0, h.stream, n, w, part_w, blocks,
+                      V + (size_t)(i + 1) * n, hc + i + 1, hc_host + i + 1));
+  count_launches(3);
+  return PMG_OK;
+}
+
 int dot(Handle &h, const double *a, const double *b, size_t n, double *result_dev) {
   PMG_CUDA(launch_pdl(k_dot, dim3(RED_BLOCKS), dim3(RED_THREADS), 0, h.stream, n, a, b, h.red_partial.p,
                       h.red_counter.p, result_dev));
