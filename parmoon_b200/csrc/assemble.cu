@@ -320,28 +320,32 @@ __global__ void __launch_bounds__(ASM_WARPS * 32, 2) k_assemble(AsmArgs a) {
   for (int base = (blockIdx.x * nw + warp) * GPW; base < a.n_elems; base += gridDim.x * nw * GPW) {
     const int e = base + grp;
     const bool valid = lane_used && e < a.n_elems;
-    if (valid) {
-      const double *cv = a.cell_vert + (size_t)e * NV * 3;
+    {
+      // (lanes without a cell of their own repeat the warp's first one; only the
+      // scratch is written under `valid`)
+      const int ec = valid ? e : base;
+      const double *cv = a.cell_vert + (size_t)ec * NV * 3;
       double J[9], x0[3], Ji[9], K[9], adet;
       cell_map<HEX>(cv, J, x0, Ji, adet, K);
-      double hconv = 0;
-      if (supg) {
-        // the reference caches the convection-direction size from the first
-        // quadrature point's b for the whole cell (ConvDiff.C:376-383)
-        double X = x0[0] + J[0] * sQ[1] + J[1] * sQ[2] + J[2] * sQ[3];
-        double Y = x0[1] + J[3] * sQ[1] + J[4] * sQ[2] + J[5] * sQ[3];
-        double Z = x0[2] + J[6] * sQ[1] + J[7] * sQ[2] + J[8] * sQ[3];
-        double c[7];
-        coeff_at(a.coef, a.ctab, NQ, e, 0, X, Y, Z, c);
-        hconv = hk_convection(HEX, a.brick != 0, cv, Ji, c[1], c[2], c[3]);
-      }
-      for (int q = t; q < NQ; q += NLOC) {
+      double c[7];
+      auto coeff_q = [&](int q) {
         const double xi = sQ[q * 4 + 1], eta = sQ[q * 4 + 2], zeta = sQ[q * 4 + 3];
         double X = x0[0] + J[0] * xi + J[1] * eta + J[2] * zeta;
         double Y = x0[1] + J[3] * xi + J[4] * eta + J[5] * zeta;
         double Z = x0[2] + J[6] * xi + J[7] * eta + J[8] * zeta;
-        double c[7];
-        coeff_at(a.coef, a.ctab, NQ, e, q, X, Y, Z, c);
+        coeff_at(a.coef, a.ctab, NQ, ec, q, X, Y, Z, c);
+      };
+      coeff_q(min(t, NQ - 1));
+      // the reference caches the convection-direction size from the first
+      // quadrature point's b for the whole cell (ConvDiff.C:376-383): it comes from
+      // the lane that evaluates that point, not from an evaluation of every lane's own
+      // (Q1 64^3 with the curl field: 404 -> 330 us)
+      const int first = lane_used ? grp * NLOC : 0;
+      const double b0 = __shfl_sync(0xffffffffu, c[1], first), b1 = __shfl_sync(0xffffffffu, c[2], first),
+                   b2 = __shfl_sync(0xffffffffu, c[3], first);
+      const double hconv = supg ? hk_convection(HEX, a.brick != 0, cv, Ji, b0, b1, b2) : 0.0;
+      for (int q = t; valid && q < NQ; q += NLOC) {
+        if (q != t) coeff_q(q);
         const double mult = sQ[q * 4] * adet;
         double delta = supg ? sdfem_delta(hconv, c[0], c[1], c[2], c[3], a.poly, a.delta0) : 0.0;
         double bh[3];  // b in reference gradients: b . (Ji^T g^) = (Ji b) . g^
