@@ -57,11 +57,11 @@ REF_BIN = os.path.join(ROOT, "oracle", "_ref", "pmg_ref")
 RESTART = 40
 N_FULL = (2 * N_CELLS + 1) ** 3
 # DRAM traffic of one FP32 SSOR step per algorithmic byte, measured with ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum over the 54 colour launches of
-# one step on the finest level of the 48^3 Q2 hierarchy: 0.858 GB for 0.663 GB
+# (dram__bytes_read.sum + dram__bytes_write.sum over the 10 launches of one step
+# on the finest level of the 48^3 Q2 hierarchy: 0.554 GB for 0.505 GB
 # algorithmic -- FP32 values, 16-bit column deltas, slice pointers, lane rows,
-# vectors); the step's traffic scales with the rows and entries it sweeps
-SSOR_TRAFFIC_PER_BYTE = 0.857810 / 0.662910
+# vectors, kept sums); the step's traffic scales with the rows and entries it sweeps
+SSOR_TRAFFIC_PER_BYTE = 0.553598 / 0.504542
 
 
 def pinned_f64(n):
@@ -500,7 +500,7 @@ def bench_ours(args, rank, world, dist):
             "fp32_solve_setup_s": statistics.mean(s.setup_seconds for s in stats),
             "fp32_vcycle_s": statistics.mean(s.vcycle_seconds for s in stats),
             "wall_s_per_step": t_wall / args.steps,
-            "roofline": {"bound": "hbm", "kernel": "k_sell_gs<float,K> (FP32 multicolour SSOR step on SELL-32, finest level)",
+            "roofline": {"bound": "hbm", "kernel": "k_sell_phase + k_sell_block (FP32 multicolour SSOR step on SELL-32, finest level)",
                          "achieved": ssor["gbs"], "peak": hbm, "unit": "GB/s", "frac": ssor["gbs"] / hbm,
                          "traffic": ssor["bytes"] * SSOR_TRAFFIC_PER_BYTE,
                          "traffic_note": "ncu DRAM bytes of one SSOR step at 48^3, scaled by the algorithmic bytes", "peak_kind": peak_kind, "bytes_per_launch": ssor["bytes"],

@@ -8,12 +8,12 @@
 //   preconditioner  TMultiGridScaIte::Iterate (src/FE/MultiGridScaIte.C:89-130)
 //   fgmres          TFgmresIte::Iterate, flexible branch (src/FE/FgmresIte.C:245-624):
 //                   right preconditioning, modified Gram-Schmidt, Givens rotations.
-//                   Dots, axpys and normalisation run on the device with the
-//                   Hessenberg entries kept in device memory; the host reads one
-//                   column per iteration for the rotations and the stop test.
+//                   Products, updates and normalisation run on the device, three
+//                   launches per column; the host reads one column per iteration
+//                   for the rotations and the stop test.
 //
 // The V-cycle is captured once per solve into a CUDA graph and replayed for
-// every preconditioner application (hundreds of small colour launches).
+// every preconditioner application (a hundred or more small launches).
 #include "pmg_internal.h"
 #include <algorithm>
 #include <cmath>
@@ -558,7 +558,7 @@ __global__ void k_prec_out32(int N, const float *__restrict__ x, double *z) {
 
 static int prepare_levels(Handle &h) {
   bool fp32 = h.prm.precision == PMG_PREC_FP32;
-  // the coarsest level's LU and inverse run on the auxiliary stream while the
+  // the coarsest level's inverse runs on the auxiliary stream while the
   // level loop below converts the SELL values on the main stream; every path
   // out of here joins the two streams first
   const bool factor = h.prm.coarse_smoother == PMG_COARSE_DIRECT && !h.coarse_ready && h.lv[0].assembled;
