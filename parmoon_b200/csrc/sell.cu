@@ -635,9 +635,11 @@ __device__ __forceinline__ void sell_load_cols(bool wd, const int *__restrict__ 
 // y = x + omega (f - A x) / a_rr (MODE 2, into a vector other than x), or the
 // defect after an SSOR step (MODE 3): the step's backward sweep has left the
 // sums over the higher colours of the final x in su, so only the lower part
-// and the diagonal are read; over slices [s0, s1)
+// and the diagonal are read.  The Dirichlet rows (slices from sd on) have no
+// colours and are read whole: a caller's matrix may hold more than the diagonal
+// there, and a transfer may take their defect to active rows.  Over slices [s0, s1)
 template <typename T, int MODE, int K>
-__global__ void __launch_bounds__(32 * K) k_sell_mv(int s0, int s1, const int *__restrict__ perm,
+__global__ void __launch_bounds__(32 * K) k_sell_mv(int s0, int s1, int sd, const int *__restrict__ perm,
                                                     const int *__restrict__ sptr, const int *__restrict__ nlow,
                                                     const int *__restrict__ col, const short *__restrict__ c16,
                                                     const unsigned char *__restrict__ wide,
@@ -663,7 +665,7 @@ __global__ void __launch_bounds__(32 * K) k_sell_mv(int s0, int s1, const int *_
   };
   auto start = [&](int sl) {
     off = __ldg(sptr + sl);
-    lmax = MODE == 3 ? __ldg(nlow + sl) + 1 : (__ldg(sptr + sl + 1) - off) >> 5;
+    lmax = MODE == 3 && sl < sd ? __ldg(nlow + sl) + 1 : (__ldg(sptr + sl + 1) - off) >> 5;
     wd = __ldg(wide + sl) != 0;
     r = __ldg(perm + sl * 32 + lane);
     load_chunk(0);
@@ -890,7 +892,7 @@ static cudaError_t launch_mv(cudaStream_t s, const Level &L, const T *x, const T
                              T omega = 0) {
   if (n < 0) n = L.sell_nslices;
   return launch_pdl(k_sell_mv<T, MODE, K>, dim3(slice_grid<T>(n, num_sms, K)), dim3(32 * K), 0, s, 0, n,
-                    (const int *)L.sell_perm.p, (const int *)L.sell_ptr.p, (const int *)L.sell_nlow.p,
+                    L.sell_group[L.sell_group.size() - 2], (const int *)L.sell_perm.p, (const int *)L.sell_ptr.p, (const int *)L.sell_nlow.p,
                     (const int *)L.sell_col.p, (const short *)L.sell_c16.p, (const unsigned char *)L.sell_wide.p,
                     sell_val<T>(L), x, f, y, sell_invd<T>(L), (const T *)sell_sum<T>(L, true), omega);
 }
