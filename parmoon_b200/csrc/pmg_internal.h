@@ -169,6 +169,7 @@ struct Level {
   // columns of lower colours, step nlow the diagonal, the rest the higher
   // ones; sell_src: an entry's position in its CSR row (SELL_NO_SRC: padding)
   bool sell_split = false;
+  bool sell_coupled = false;  // two rows of one colour are coupled (then not split either)
   DBuf<int> sell_nlow;
   DBuf<unsigned short> sell_src;
   DBuf<float> sell_sl32, sell_su32;  // sums over the lower / higher colours kept between sweeps

@@ -158,8 +158,9 @@ static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std:
 // entries of each row in the solve copy: an active row keeps its columns < Na
 // (columns are sorted, so that is a prefix), a Dirichlet row all of its own;
 // nlow: those of lower colours, ins: those of lower / higher colours of the same
-// phase (16 + 16 bits, saturated).  bad: two rows of one colour are coupled, or a
-// row is too long for the 16-bit source index.
+// phase (16 + 16 bits, saturated).  bad: two rows of one colour are coupled
+// (BAD_COUPLED), a row is too long for the 16-bit source index (BAD_LONG).
+enum { BAD_COUPLED = 1, BAD_LONG = 2 };
 __global__ void k_row_counts(int N, int Na, const int *__restrict__ rp, const int *__restrict__ kc,
                              const int *__restrict__ colour, const int *__restrict__ phase, int *__restrict__ alen,
                              int *__restrict__ nlow, unsigned *__restrict__ ins, int *bad) {
@@ -189,9 +190,10 @@ __global__ void k_row_counts(int N, int Na, const int *__restrict__ rp, const in
     } else {
       n = e - b;
     }
-    if (__any_sync(0xffffffffu, same) && lane == 0) *bad = 1;
+    same = __any_sync(0xffffffffu, same);
     if (lane == 0) {
-      if (n >= SELL_NO_SRC) *bad = 1;
+      if (same) atomicOr(bad, BAD_COUPLED);
+      if (n >= SELL_NO_SRC) atomicOr(bad, BAD_LONG);
       alen[r] = n;
       nlow[r] = low;
       ins[r] = (unsigned)min(li, 65535) | (unsigned)min(ui, 65535) << 16;
@@ -484,6 +486,7 @@ int build_sell(Handle &h, Level &L) {
   L.sell_nslices = nslices;
   L.sell_nnz = total;
   L.sell_split = split;
+  L.sell_coupled = (bad & BAD_COUPLED) != 0;
   L.sell_nnz_narrow = (long)nnz[0];
   L.sell_nnz_wide = (long)nnz[1];
   L.sell_ready = true;
@@ -1376,7 +1379,8 @@ static int sweep_colours(cudaStream_t s, const Level &L, bool forward, int mode,
 // to each other), so the second of two successive updates of a colour is left
 // out where the sweeps turn.  (The skipped passes' sums stay right: the last
 // colour has no higher colours and the first no lower ones, so theirs are
-// always 0.)
+// always 0.)  Where two rows of one colour are coupled (sell_coupled) a repeated
+// update does change x, and none is left out.
 //
 // By blocks, one phase is a product over the whole GPU for what comes from
 // outside and one launch for the phase's own colours: 27 colours in 3 phases are 8
@@ -1391,7 +1395,7 @@ int sell_ssor(cudaStream_t s, const Level &L, const T *f, T *x, double omega, in
               int *err) {
   const T om = (T)omega;
   if (!use_blocks<T>(L)) {
-    const int skip = omega == 1.0 ? 1 : 0;
+    const int skip = omega == 1.0 && !L.sell_coupled ? 1 : 0;
     for (int k = 0; k < steps; k++) {
       const int fwd = !L.sell_split || (k == 0 && start == SWEEP_ANY) ? GS_FULL
                       : k == 0                                        ? GS_LOWER_ZERO
