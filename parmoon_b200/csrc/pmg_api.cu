@@ -761,9 +761,10 @@ int pmg_time_kernel(pmg_handle hh, int kernel, int level, int form, int reps, do
     fl = kernel == PMG_KERNEL_SPMV32 ? 2 * nnz : 4 * nnz;
   } else if (kernel == PMG_KERNEL_COARSE_FACTOR) {
     if (level != 0) { set_error("pmg_time_kernel: the coarse factorisation is of level 0"); return PMG_ERR_ARG; }
-    // the inverse by exchange steps takes 2 n^3 flops; the dense matrix is read and written
+    // the inverse by exchange steps takes 2 n^3 flops, its Newton step as many; the
+    // dense matrix is read and written
     by = 2.0 * 8.0 * N * N;
-    fl = 2.0 * N * N * N;
+    fl = 4.0 * N * N * N;
   } else if (kernel == PMG_KERNEL_LEARNED_FWD) {
     if (!h->has_learned || L.lat_n[0] <= 0) {
       set_error("pmg_time_kernel: the learned forward needs weights and the level's lattice");

@@ -238,7 +238,8 @@ struct Handle {
   int device = 0;
   int num_sms = 148;
   // coarsest-level dense inverse (FP64)
-  DBuf<double> coarse_lu, coarse_w, coarse_inv, coarse_t;  // active block: work array, pivot rows, inverse; reduced rhs
+  // active block: work array, pivot rows, inverse before and after its Newton step; reduced rhs
+  DBuf<double> coarse_lu, coarse_w, coarse_x, coarse_inv, coarse_t;
   DBuf<int> coarse_piv, coarse_perm;  // pivot row of each column, column of each row
   DBuf<int> coarse_cptr;  // colour pointers of the coarsest level's rows (iterative coarse solve)
   bool coarse_ready = false;

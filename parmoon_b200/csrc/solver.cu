@@ -35,11 +35,13 @@ int level_invdiag(cudaStream_t s, Level &L, int *flags);
 //   k_gj_update  the other columns, for all rows at once: M_i := (0 for a pivot
 //                row, M_i otherwise) + panel_i W
 //   k_gj_finish  the permutation
+//   k_inv_residual, k_inv_refine  one Newton step (below)
 // n / 24 panels of two launches replace an LU (panels in shared memory, row
 // swaps, triangular solves, updates) and a substitution pass for the inverse:
-// n = 729 1.5 ms against 3.5 ms before (23 panels of 60 us, inverse 1.26 ms).  A step
-// is bound by its two CTA barriers, the pivot's reduction and one division (1.7
-// us; a rolled loop, and a search beside the update, were no faster).
+// n = 729 1.44 ms and 0.12 ms for the Newton step, against 3.43 ms (23 panels of 60
+// us, inverse 1.26 ms).  An exchange step is bound by its two CTA barriers, the
+// pivot's reduction and one division (1.7 us; a rolled loop, and a search beside
+// the update, were no faster).
 constexpr int GJ_NB = 24, GJ_MAX_N = 832;  // one thread per row: 26 warps, 78 registers
 
 __global__ void __launch_bounds__(GJ_MAX_N, 1) k_gj_panel(int n, int k0, double *__restrict__ M, double *__restrict__ W,
@@ -154,6 +156,125 @@ __global__ void k_gj_finish(int n, const double *__restrict__ M, const int *__re
   for (int k = threadIdx.x; k < n; k += blockDim.x) Inv[(size_t)j * n + piv[k]] = row[k];
 }
 
+// One Newton step X + X (I - A X) after the exchange steps: these alone leave 1.3
+// to 1.6 times the error of an LU with substitution, the step brings it below
+// that (what is left is the rounding of X).  A X from the sparse rows, in twice the
+// working precision (exact products by FMA, sums with their rounding errors kept),
+// because the residual is all rounding; X R in FP64.  norm: the largest row sum of
+// |R|; from 1/2 on (a matrix singular to working precision) the step could do harm
+// and X stays as it is.  729 rows: 50 us (bound by its 8 FP64 operations per term) and
+// 71 us; launched without programmatic dependence, whose waiting CTAs cost 120 us more.
+__global__ void __launch_bounds__(256) k_inv_residual(int n, const int *__restrict__ rp, const int *__restrict__ kc,
+                                                      const double *__restrict__ a, const double *__restrict__ X,
+                                                      double *__restrict__ R, unsigned long long *norm) {
+  constexpr int J = (GJ_MAX_N + 255) / 256, ROW = 256;  // columns per thread; entries staged at a time
+  __shared__ double sh[8], sv[ROW];
+  __shared__ int sc[ROW];
+  pdl_wait();
+  pdl_trigger();
+  const int i = blockIdx.x, end = __ldg(rp + i + 1), j0 = threadIdx.x;
+  double s[J], c[J];
+#pragma unroll
+  for (int u = 0; u < J; u++) {
+    s[u] = i == j0 + 256 * u ? 1.0 : 0.0;
+    c[u] = 0.0;
+  }
+  for (int k0 = __ldg(rp + i); k0 < end; k0 += ROW) {
+    const int m = min(ROW, end - k0);
+    if (j0 < m) {
+      const int col = __ldg(kc + k0 + j0);
+      sc[j0] = col < n ? col : 0;  // (a Dirichlet column: 0 times any row of X)
+      sv[j0] = col < n ? -__ldg(a + k0 + j0) : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < m; k++) {
+      const double v = sv[k], *x = X + (size_t)sc[k] * n + j0;
+#pragma unroll
+      for (int u = 0; u < J; u++) {
+        const double xu = j0 + 256 * u < n ? x[256 * u] : 0.0, p = v * xu, t = s[u] + p, z = t - s[u];
+        c[u] += ((s[u] - (t - z)) + (p - z)) + fma(v, xu, -p);
+        s[u] = t;
+      }
+    }
+    __syncthreads();
+  }
+  double sum = 0.0;
+#pragma unroll
+  for (int u = 0; u < J; u++) {
+    s[u] += c[u];
+    if (j0 + 256 * u < n) {
+      R[(size_t)i * n + j0 + 256 * u] = s[u];
+      sum += fabs(s[u]);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) sum += sh[w];
+    // (the bits of non-negative doubles are ordered as the doubles, NaN above all)
+    atomicMax(norm, (unsigned long long)__double_as_longlong(fabs(sum)));
+  }
+}
+
+// 64 x 32 tiles, 4 x 2 per thread (729 rows: 276 tiles for 148 SMs), 16 columns of X and
+// rows of R at a time by cp.async, the next ones on their way meanwhile
+__device__ __forceinline__ void cp_async8(double *dst, const double *src, bool on) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(on ? 8 : 0)
+               : "memory");
+}
+__global__ void __launch_bounds__(256) k_inv_refine(int n, const double *__restrict__ X, const double *__restrict__ R,
+                                                    const unsigned long long *norm, double *__restrict__ out) {
+  constexpr int BK = 16;
+  __shared__ double Xs[2][64][BK + 1], Rs[2][BK][32];
+  pdl_wait();
+  pdl_trigger();
+  const bool on = __longlong_as_double((long long)*norm) < 0.5;
+  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 32, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  double s[4][2] = {};
+  auto load = [&](int k0, int buf) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const bool in = r0 + ty + 16 * q < n && k0 + tx < n;
+      cp_async8(&Xs[buf][ty + 16 * q][tx], X + (in ? (size_t)(r0 + ty + 16 * q) * n + k0 + tx : 0), in);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const bool in = k0 + ty < n && c0 + tx + 16 * q < n;
+      cp_async8(&Rs[buf][ty][tx + 16 * q], R + (in ? (size_t)(k0 + ty) * n + c0 + tx + 16 * q : 0), in);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  if (on) {
+    load(0, 0);
+    for (int k0 = 0, buf = 0; k0 < n; k0 += BK, buf ^= 1) {
+      if (k0 + BK < n) {
+        load(k0 + BK, buf ^ 1);
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < BK; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 2; j++) s[i][j] += Xs[buf][ty + 16 * i][k] * Rs[buf][k][tx + 16 * j];
+      __syncthreads();  // the buffer is read before it is filled again
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
+      if (r < n && c < n) out[(size_t)r * n + c] = X[(size_t)r * n + c] + s[i][j];
+    }
+}
+
 // the coarsest level's rhs reduced to its active rows: t = f_a - A_ad f_d
 // (rows >= Na are Dirichlet: x_d = f_d); one warp per row
 template <typename T>
@@ -219,6 +340,7 @@ static int coarse_factor_launch(Handle &h, cudaStream_t s) {
     return PMG_OK;
   }
   PMG_TRY(h.coarse_lu.alloc((size_t)n * n));
+  PMG_TRY(h.coarse_x.alloc((size_t)n * n));
   PMG_TRY(h.coarse_inv.alloc((size_t)n * n));
   PMG_TRY(h.coarse_w.alloc((size_t)GJ_NB * n));
   PMG_TRY(h.coarse_piv.alloc(n));
@@ -236,8 +358,12 @@ static int coarse_factor_launch(Handle &h, cudaStream_t s) {
     count_launches(2);
   }
   PMG_CUDA(launch_pdl(k_gj_finish, dim3(n), dim3(256), 0, s, n, (const double *)M, (const int *)h.coarse_piv.p,
-                      h.coarse_inv.p));
-  count_launches(2);
+                      h.coarse_x.p));
+  unsigned long long *norm = reinterpret_cast<unsigned long long *>(h.coarse_flags.p + 2);
+  k_inv_residual<<<n, 256, 0, s>>>(n, L.rowptr.p, L.kcol.p, L.A.p, h.coarse_x.p, M, norm);
+  k_inv_refine<<<dim3(tiles, (n + 63) / 64), 256, 0, s>>>(n, h.coarse_x.p, M, norm, h.coarse_inv.p);
+  PMG_CUDA(cudaGetLastError());
+  count_launches(4);
   PMG_CUDA(cudaMemcpyAsync(h.h_coarse_flags, h.coarse_flags.p, sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
   return PMG_OK;
 }
