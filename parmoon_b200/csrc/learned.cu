@@ -134,12 +134,21 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// D = A B, the first of a chain
+__device__ __forceinline__ void mma_bf16_first(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%10,%10,%10};\n"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+
 // CONV_HIDDEN: xo = ReLU(conv + b) as BF16.
 // CONV_STENCIL: the stencil W[co][L] = (conv + b)[co] * dscale[L], co < cout.
 // CONV_GRAD: the data gradient: the input is a gradient in three BF16 parts
 //   (accumulated one after the other), xo gets conv * (act > 0) in three parts, and
 //   bsum[CTA][32] the CTA's sums of it per channel (the bias gradient's partials).
-//   0.22 ms per 32 x 32 layer at 65^3 nodes (FP32 CUDA cores before: 0.81 ms).
+//   0.24 ms per 32 x 32 layer at 65^3 nodes (FP32 CUDA cores before: 0.81 ms).
 enum { CONV_HIDDEN = 0, CONV_STENCIL = 1, CONV_GRAD = 2 };
 template <int MODE>
 __global__ void __launch_bounds__(256, 2)
@@ -176,15 +185,29 @@ __global__ void __launch_bounds__(256, 2)
   for (int br = blockIdx.x; br < nbricks; br += gridDim.x) {
     const int bx = br % nbx, by = (br / nbx) % nby, bz = br / (nbx * nby);
     const int x0 = bx * CONV_BX, y0 = by * CONV_BY, z0 = bz * CONV_BZ;
-    float acc[2][4][4];
+    float acc[2][4][4], tot[GRAD ? 2 : 1][4][4];
 #pragma unroll
     for (int m = 0; m < 2; m++)
 #pragma unroll
       for (int nt = 0; nt < 4; nt++)
 #pragma unroll
-        for (int e = 0; e < 4; e++) acc[m][nt][e] = 0.0f;
-    // (the smallest part first: the tensor cores round every sum towards zero, and
-    // relative to a small sum that is little)
+        for (int e = 0; e < 4; e++) acc[m][nt][e] = tot[GRAD ? m : 0][nt][e] = 0.0f;
+    // The tensor cores round every sum towards zero.  The gradient's smallest part
+    // comes first (relative to a small sum that is little); the leading part's sums
+    // leave the accumulators after every offset (2 mma) for FP32 sums in registers,
+    // which round to nearest.  Without that the gradients of the first two layers
+    // were 2 to 3 times as far from FP64 as with FP32 arithmetic throughout.
+    auto flush = [&]() {
+#pragma unroll
+      for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            tot[GRAD ? m : 0][nt][e] += acc[m][nt][e];
+            acc[m][nt][e] = 0.0f;
+          }
+    };
     for (int part = GRAD ? 2 : 0; part >= 0; part--) {
       const __nv_bfloat16 *xp = xi + part * NL * 32;
       __syncthreads();  // the previous reads of the halo are done
@@ -224,8 +247,17 @@ __global__ void __launch_bounds__(256, 2)
               mma_bf16(acc[m][2 * p + 1], a[m], b[p][2], b[p][3]);
             }
         }
+        if (GRAD && part == 0) flush();
       }
+      if (GRAD && part > 0) flush();
     }
+    if (GRAD)
+#pragma unroll
+      for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) acc[m][nt][e] = tot[GRAD ? m : 0][nt][e];
     // epilogue: c0,c1 = (row g, channels 2q, 2q+1), c2,c3 = (row g+8, ...)
     const int g = lane >> 2, q = lane & 3;
     const int gy = y0 + warp;
@@ -279,9 +311,9 @@ __global__ void __launch_bounds__(256, 2)
       }
     __syncthreads();
     if (tid < 32) {
-      float v = 0.0f;
+      double v = 0.0;
       for (int w = 0; w < 8; w++) v += sb[w * 32 + tid];
-      bsum[blockIdx.x * 32 + tid] = v;
+      bsum[blockIdx.x * 32 + tid] = (float)v;
     }
   }
 }
@@ -294,16 +326,18 @@ __global__ void __launch_bounds__(256, 2)
 // next brick on its way by cp.async meanwhile.  18 warps: warp w holds the
 // accumulators of offsets 3 (w % 9) .. + 2 for 16 of the 32 channels co; per 16
 // nodes 3 + 6 ldmatrix.x4 feed 36 mma.  The tensor cores round their sums towards
-// zero, so after every WG_FLUSH runs of 16 nodes (6 mma) a thread adds its accumulators
-// to FP32 sums of its own in shared memory and starts from 0 again.  One CTA per
+// zero, so nothing stays in them: the leading parts' products of 16 nodes are one
+// mma from 0 (their sum mostly fits 24 bits), the two smaller parts' a chain of two,
+// and both are added to FP32 sums in registers, which go to sums of their own in
+// shared memory after every brick.  One CTA per
 // SM; every CTA leaves its sums in part[CTA] and k_wgrad_sum adds those in order,
 // so the result does not depend on the schedule.
-// At 65^3 nodes 0.20 ms per layer (46 GFLOP in three parts, bound by the mma.sync
+// At 65^3 nodes 0.23 ms per layer (46 GFLOP in three parts, bound by the mma.sync
 // and ldmatrix issue rate); the FP32 kernel before it read dz once per (ci, k)
-// through L2, 864 times in all, and took 5.4 ms.  Against FP64 the gradient is
-// as far off as with that kernel (1.0002 times on average over lattices of 9 to
-// 65 nodes a side; without taking the sums out 1.06 times at 65).
-constexpr int WG_WARPS = 18, WG_NODES = CONV_BX * CONV_BY, WG_HALO = CONV_HX * CONV_HY * 3, WG_FLUSH = 2;
+// through L2, 864 times in all, and took 5.4 ms.  The error against FP64 with the
+// same activations is 4e-8 to 7e-8 of the gradient (8 to 32 cells a side), with the
+// FP32 kernel 6e-8 to 1.2e-7.
+constexpr int WG_WARPS = 18, WG_NODES = CONV_BX * CONV_BY, WG_HALO = CONV_HX * CONV_HY * 3;
 constexpr int WG_STAGE = (WG_HALO + 3 * WG_NODES) * 64;  // 59,136 bytes, two stages
 constexpr int WG_SMEM = 2 * WG_STAGE + 48 * 32 * WG_WARPS * (int)sizeof(float);
 __device__ __forceinline__ void ldsm_x4_t(unsigned addr, unsigned (&r)[4]) {
@@ -386,24 +420,36 @@ __global__ void __launch_bounds__(32 * WG_WARPS, 1)
         for (int p = 0; p < 2; p++) {
           unsigned b[4];
           ldsm_x4_t(s_x + swz(row, 2 * p + b_ch), b);
+          float t[2][4];
 #pragma unroll
-          for (int q = 2; q >= 0; q--) {
-            mma_bf16(acc[o][2 * p], a[q], b[0], b[1]);
-            mma_bf16(acc[o][2 * p + 1], a[q], b[2], b[3]);
+          for (int q = 1; q >= 0; q--) {
+            if (q) {
+              mma_bf16_first(t[0], a[2], b[0], b[1]);
+              mma_bf16_first(t[1], a[2], b[2], b[3]);
+              mma_bf16(t[0], a[1], b[0], b[1]);
+              mma_bf16(t[1], a[1], b[2], b[3]);
+            } else {
+              mma_bf16_first(t[0], a[0], b[0], b[1]);
+              mma_bf16_first(t[1], a[0], b[2], b[3]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              acc[o][2 * p][e] += t[0][e];
+              acc[o][2 * p + 1][e] += t[1][e];
+            }
           }
         }
       }
-      if (ks % WG_FLUSH != WG_FLUSH - 1) continue;
-#pragma unroll
-      for (int o = 0; o < 3; o++)
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            own[((o * 4 + nt) * 4 + e) * 32 * WG_WARPS] += acc[o][nt][e];
-            acc[o][nt][e] = 0.0f;
-          }
     }
+#pragma unroll
+    for (int o = 0; o < 3; o++)
+#pragma unroll
+      for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          own[((o * 4 + nt) * 4 + e) * 32 * WG_WARPS] += acc[o][nt][e];
+          acc[o][nt][e] = 0.0f;
+        }
     __syncthreads();  // this brick's reads are done before its buffer is filled again
   }
   const int g = lane >> 2, q = lane & 3;
@@ -424,12 +470,12 @@ __global__ void __launch_bounds__(32 * WG_WARPS, 1)
 __global__ void __launch_bounds__(256) k_wgrad_sum(int cin, int cout, int nw, const float *__restrict__ part, int nb,
                                                    const float *__restrict__ bsum, float *__restrict__ gw,
                                                    float *__restrict__ gb) {
-  __shared__ float run[4][64];
+  __shared__ double run[4][64];
   const int t = blockIdx.x * 64 + (threadIdx.x & 63), q = threadIdx.x >> 6;
   const bool weight = t < 27 * 1024;
   const int n = weight ? nw : nb, stride = weight ? 27 * 1024 : 32;
   const float *src = weight ? part + t : bsum + (t - 27 * 1024);
-  float v = 0.0f;
+  double v = 0.0;
   if (weight || t < 27 * 1024 + 32) {
     const int per = (n + 3) / 4, c1 = min(n, (q + 1) * per);
 #pragma unroll 8
@@ -441,9 +487,9 @@ __global__ void __launch_bounds__(256) k_wgrad_sum(int cin, int cout, int nw, co
   v = (run[0][threadIdx.x] + run[1][threadIdx.x]) + (run[2][threadIdx.x] + run[3][threadIdx.x]);
   if (weight) {
     const int k = t >> 10, co = t >> 5 & 31, ci = t & 31;
-    if (co < cout && ci < cin) gw[((size_t)co * cin + ci) * 27 + k] += v;
+    if (co < cout && ci < cin) gw[((size_t)co * cin + ci) * 27 + k] += (float)v;
   } else if (t < 27 * 1024 + cout) {
-    gb[t - 27 * 1024] += v;
+    gb[t - 27 * 1024] += (float)v;
   }
 }
 
@@ -622,9 +668,9 @@ __global__ void __launch_bounds__(256) k_train_dout(int n1, const float *__restr
   for (int e = 0; e < 8; e++) sb[threadIdx.x >> 2][c8 * 8 + e] = bs[e];
   __syncthreads();
   if (threadIdx.x < 32) {
-    float v = 0.0f;
+    double v = 0.0;
     for (int w = 0; w < 64; w++) v += sb[w][threadIdx.x];
-    bsum[blockIdx.x * 32 + threadIdx.x] = v;
+    bsum[blockIdx.x * 32 + threadIdx.x] = (float)v;
   }
 }
 
