@@ -90,10 +90,12 @@ __global__ void k_pack_weights_t(int cin, int cout, const __nv_bfloat16 *__restr
   wpk[t] = (co < cout && ci < cin) ? w[((size_t)co * cin + ci) * 27 + 26 - k] : __float2bfloat16(0.0f);
 }
 
-// v = h + m + l, three BF16 numbers (exact: 3 x 8 significant bits, up to underflow)
+// v = h + m + l, three BF16 numbers (exact: 3 x 8 significant bits, up to
+// underflow).  An infinite v is h = v alone (v - h would be NaN), and the values
+// that round to infinity in BF16 although finite are cut off instead.
 __device__ __forceinline__ void split3(float v, __nv_bfloat16 &h, __nv_bfloat16 &m, __nv_bfloat16 &l) {
-  h = __float2bfloat16(v);
-  const float r = v - __bfloat162float(h);
+  h = fabsf(v) < 0x1.fep127f ? __float2bfloat16_rn(v) : __float2bfloat16_rz(v);
+  const float r = isfinite(v) ? v - __bfloat162float(h) : 0.0f;
   m = __float2bfloat16(r);
   l = __float2bfloat16(r - __bfloat162float(m));
 }
