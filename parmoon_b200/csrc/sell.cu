@@ -1090,6 +1090,7 @@ struct BlkArgs {
   T *x, *sl, *su;
   T omega;
   int *err;
+  int extra;  // added to what every wait expects (PMG_TEST_BLK_EXTRA)
 };
 
 // four steps of a lane: values and slots
@@ -1163,7 +1164,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_sell_block(const __grid_constant_
     int p = h - 1;
     while (p >= 0 && slices(p) == 0) p--;
     dep[h] = p < 0 ? NO_DEP : p;
-    need[h] = slices(h);
+    need[h] = slices(h) + a.extra;
     done[h] = 0;
   }
   __syncthreads();
@@ -1339,6 +1340,11 @@ static int launch_block(cudaStream_t st, const Level &L, int p, const T *f, T *x
   a.su = sell_sum<T>(L, true);
   a.omega = omega;
   a.err = err;
+  // PMG_TEST_BLK_EXTRA=<n>: every wait expects n slices that nobody does, so it runs
+  // out -- the test of the give-up path (read at every launch; a captured V-cycle
+  // graph keeps the value it was captured with)
+  const char *extra = getenv("PMG_TEST_BLK_EXTRA");
+  a.extra = extra ? std::max(0, atoi(extra)) : 0;
   const int nb = L.blk_n[p];
   // 16 warps with every row's chunks in registers while a block has few slices,
   // and in FP64 always (registers); 32 warps with 4 chunks for the larger blocks
