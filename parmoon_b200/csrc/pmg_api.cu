@@ -796,6 +796,8 @@ int pmg_time_kernel(pmg_handle hh, int kernel, int level, int form, int reps, do
   PMG_CUDA(cudaEventSynchronize(h->ev[5]));
   float ms = 0;
   PMG_CUDA(cudaEventElapsedTime(&ms, h->ev[4], h->ev[5]));
+  // (a sweep whose wait gave up is no measurement, and its flag is not the next solve's)
+  if (kernel == PMG_KERNEL_SSOR64 || kernel == PMG_KERNEL_SSOR32) PMG_TRY(coarse_cycle_check(*h));
   *sec = ms * 1e-3 / reps;
   if (bytes) *bytes = by;
   if (flops) *flops = fl;

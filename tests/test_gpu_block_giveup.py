@@ -46,3 +46,18 @@ def test_solve_gives_up_and_recovers(prec):
     r = run(prec, SOLVE)
     assert r["rc_fail"] == -3, r
     assert r["rc_ok"] == 0 and r["rel"] <= 1e-10, r
+
+
+TIMED = r"""
+sec = ctypes.c_double()
+rc_fail = P.lib().pmg_time_kernel(h.h, {kernel}, 1, P.FORM_SUPG, 1, ctypes.byref(sec), None, None)
+"""
+
+
+@pytest.mark.parametrize("prec,kernel", [(0, 2), (1, 3)])
+def test_timed_sweep_reports_and_clears(prec, kernel):
+    """pmg_time_kernel runs the same sweeps: it reports what gave up, and leaves no
+    flag behind for the next solve."""
+    r = run(prec, TIMED.format(kernel=kernel))
+    assert r["rc_fail"] == -3, r
+    assert r["rc_ok"] == 0 and r["rel"] <= 1e-10, r
