@@ -1124,11 +1124,7 @@ static int launch_assemble(Handle &h, Level &L, AsmArgs a) {
     return PMG_ERR_UNSUPPORTED;
   }
   size_t smem = sizeof(double) * (fixed + (size_t)warps * per_warp);
-  static bool attr_set = false;
-  if (!attr_set) {
-    PMG_CUDA(cudaFuncSetAttribute(k_assemble<E, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    attr_set = true;
-  }
+  PMG_CUDA(func_smem(k_assemble<E, NQ>, 227 * 1024));
   h.asm_path = 3;
   int per_block = warps * GPW;
   const int *ed0 = a.elem_dof;
@@ -1158,12 +1154,8 @@ template <int E, int NQ>
 static int launch_assemble_cc(Handle &h, Level &L, AsmArgs a, const double *stab) {
   constexpr int NLOC = ET<E>::NLOC;
   const size_t smem = sizeof(double) * (16 * (size_t)NLOC * NLOC + (size_t)ASMC_WARPS * ASMC_P * (33 + NQ));
-  static bool attr_set = false;
-  if (!attr_set) {
-    PMG_CUDA(cudaFuncSetAttribute(k_assemble_cc<E, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PMG_CUDA(cudaFuncSetAttribute(k_assemble_cc<E, NQ>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    attr_set = true;
-  }
+  PMG_CUDA(func_smem(k_assemble_cc<E, NQ>, smem));
+  PMG_CUDA(func_attr((const void *)k_assemble_cc<E, NQ>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   h.asm_path = 2;
   const int per_block = ASMC_WARPS * ASMC_P;
   const int *ed0 = a.elem_dof;
@@ -1189,9 +1181,9 @@ template <int E, int KS>
 static int launch_contract(Handle &h, Level &L, AsmArgs a, const double *tfrag) {
   constexpr int NLOC = ET<E>::NLOC, NN = NLOC * NLOC, MT = (NN + 7) / 8, NB = (MT + 7) / 8, WARPS = 16;
   const size_t smem = sizeof(double) * (size_t)MT * KS * 32;
+  PMG_CUDA(func_smem(k_assemble_tc16<E, KS>, smem));
   static int per_sm = 0;  // resident blocks per SM: the grid never exceeds one wave
   if (!per_sm) {
-    PMG_CUDA(cudaFuncSetAttribute(k_assemble_tc16<E, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     PMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_assemble_tc16<E, KS>, WARPS * 32, smem));
     if (per_sm < 1) per_sm = 1;
   }

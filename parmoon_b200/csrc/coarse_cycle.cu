@@ -497,11 +497,11 @@ template <> const double *lv_p<double>(const Level &L, bool r) { return r ? L.rv
 
 template <typename T>
 static int cluster_ctas() {
+  const void *kernel = (const void *)k_coarse_cycle<T>;
+  func_attr(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  func_attr(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CC_SMEM_X);
   static int ctas = 0;
   if (ctas) return ctas;
-  const void *kernel = (const void *)k_coarse_cycle<T>;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CC_SMEM_X);
   for (int want : {16, 8, 4}) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(want);
@@ -675,13 +675,7 @@ int coarse_cycle(Handle &h, int top) {
   a.omega = (T)h.prm.smooth_omega;
   a.damp = (T)h.prm.gmg_damp;
   const int ctas = h.cc_ctas;
-  if (ctas == 1) {
-    static bool attr = false;
-    if (!attr) {
-      PMG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CC_SMEM_X));
-      attr = true;
-    }
-  }
+  if (ctas == 1) PMG_CUDA(func_smem(k_coarse_cycle<T>, CC_SMEM_X));
   if (smem > CC_SMEM_X) {
     set_error("coarse_cycle: iterates exceed the shared-memory budget");
     return PMG_ERR_ARG;

@@ -530,13 +530,10 @@ template int learned_smooth<double>(cudaStream_t, const Level &, const double *,
 
 // ------------------------------------------------------------- network driver
 static int set_conv_attrs() {
-  static bool done = false;
-  if (done) return PMG_OK;
-  PMG_CUDA(cudaFuncSetAttribute(k_conv_tc<CONV_HIDDEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM));
-  PMG_CUDA(cudaFuncSetAttribute(k_conv_tc<CONV_STENCIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM));
-  PMG_CUDA(cudaFuncSetAttribute(k_conv_tc<CONV_GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM));
-  PMG_CUDA(cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM));
-  done = true;
+  PMG_CUDA(func_smem(k_conv_tc<CONV_HIDDEN>, CONV_SMEM));
+  PMG_CUDA(func_smem(k_conv_tc<CONV_STENCIL>, CONV_SMEM));
+  PMG_CUDA(func_smem(k_conv_tc<CONV_GRAD>, CONV_SMEM));
+  PMG_CUDA(func_smem(k_conv_wgrad, WG_SMEM));
   return PMG_OK;
 }
 

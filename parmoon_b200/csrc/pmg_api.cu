@@ -6,6 +6,7 @@
 // reference exits on bad input; this library returns PMG_ERR_*).
 #include "pmg_internal.h"
 #include "fe_tables.h"
+#include "func_attr.h"
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -23,6 +24,16 @@ void set_error(const std::string &msg) { g_err = msg; }
 static std::atomic<unsigned long long> g_launches{0};
 void count_launches(unsigned long long n) { g_launches += n; }
 unsigned long long launches_so_far() { return g_launches.load(); }
+
+cudaError_t func_attr(const void *fn, cudaFuncAttribute attr, int value) {
+  static FuncAttrs known;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  e = (cudaError_t)known.once(fn, (int)attr, device, value, [&] { return cudaFuncSetAttribute(fn, attr, value); });
+  if (e != cudaSuccess) cudaGetLastError();  // (returned here; not the next launch's error)
+  return e;
+}
 
 int level_invdiag(cudaStream_t s, Level &L, int *flags);
 

@@ -60,6 +60,13 @@ static inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 blo
 }
 #endif
 
+// a kernel's attribute on the current device (func_attr.h)
+cudaError_t func_attr(const void *fn, cudaFuncAttribute attr, int value);
+template <typename... KArgs>
+static inline cudaError_t func_smem(void (*kern)(KArgs...), size_t bytes) {
+  return func_attr((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 // ------------------------------------------------------------- device buffers
 template <typename T>
 struct DBuf {

@@ -1305,12 +1305,7 @@ static int launch_phase(cudaStream_t st, const Level &L, int p, const T *f, cons
 
 template <typename T, int W, int NC, int DIR, bool TURN, int SRC, bool PLAIN>
 static int launch_block_k(cudaStream_t st, const BlkArgs<T> &a, int blocks, size_t smem) {
-  static bool attr = false;
-  if (!attr) {
-    PMG_CUDA(cudaFuncSetAttribute(k_sell_block<T, W, NC, DIR, TURN, SRC, PLAIN>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BLK_SMEM));
-    attr = true;
-  }
+  PMG_CUDA(func_smem(k_sell_block<T, W, NC, DIR, TURN, SRC, PLAIN>, BLK_SMEM));
   PMG_CUDA(launch_pdl(k_sell_block<T, W, NC, DIR, TURN, SRC, PLAIN>, dim3(blocks), dim3(32 * W), smem, st, a));
   count_launches(1);
   return PMG_OK;
