@@ -748,7 +748,7 @@ int pmg_time_kernel(pmg_handle hh, int kernel, int level, int form, int reps, do
     PMG_TRY(fill(s, x64.p, 1.0, L.N)); PMG_TRY(fill(s, y64.p, 1.0, L.N));
     double spmv_b = 12 * nnz + 4 * (N + 1) + 16 * N;  // CSR: values + columns + row pointers + x once + y
     if (kernel != PMG_KERNEL_CSR_SPMV64) {
-      PMG_TRY(sell_values<double>(*h, L));
+      PMG_TRY(kernel == PMG_KERNEL_SSOR64 ? sell_sweep_values<double>(*h, L, true) : sell_values<double>(*h, L));
       // SELL: values + column deltas / columns + slice pointers + row of each lane + x once + y
       spmv_b = 8.0 * (L.sell_nnz_narrow + L.sell_nnz_wide) + 2.0 * L.sell_nnz_narrow + 4.0 * L.sell_nnz_wide +
                4.0 * (L.sell_nslices + 1) + 4 * N + 16 * N;
@@ -760,7 +760,7 @@ int pmg_time_kernel(pmg_handle hh, int kernel, int level, int form, int reps, do
       by += spmv_b + 16 * N - (L.sell_split ? 0.5 * (10.0 * L.sell_nnz_narrow + 12.0 * L.sell_nnz_wide) : 0.0);
     fl = kernel == PMG_KERNEL_SSOR64 ? 4 * nnz : 2 * nnz;
   } else if (kernel == PMG_KERNEL_SPMV32 || kernel == PMG_KERNEL_SSOR32) {
-    PMG_TRY(sell_values<float>(*h, L));
+    PMG_TRY(kernel == PMG_KERNEL_SSOR32 ? sell_sweep_values<float>(*h, L, true) : sell_values<float>(*h, L));
     PMG_TRY(x32.alloc(L.N)); PMG_TRY(y32.alloc(L.N));
     PMG_CUDA(cudaMemsetAsync(x32.p, 0, sizeof(float) * L.N, s));
     PMG_CUDA(cudaMemsetAsync(y32.p, 0, sizeof(float) * L.N, s));

@@ -193,6 +193,7 @@ struct Level {
   long blk_chunks = 0;         // chunks of 4 steps of the inside entries
   DBuf<float> blk_val32;       // their values in that layout
   DBuf<double> blk_val64;
+  bool blk_val_fresh32 = false, blk_val_fresh64 = false;  // hold the solve copy's present values
   DBuf<float> sell_base32;   // f minus the sums from outside the block (slice order)
   DBuf<double> sell_base64;
   long sell_nnz_narrow = 0, sell_nnz_wide = 0;  // stored entries with 16-bit / 32-bit columns
@@ -339,6 +340,9 @@ int check_finite(cudaStream_t s, const double *x, size_t n, int *flag);
 int build_sell(Handle &h, Level &L);
 template <typename T>
 int sell_values(Handle &h, Level &L);
+// the values and what SOR sweeps (ssor: SSOR steps) need beside them
+template <typename T>
+int sell_sweep_values(Handle &h, Level &L, bool ssor);
 template <typename T>
 int sell_spmv(cudaStream_t s, const Level &L, const T *x, const T *f, T *y, int mode, int num_sms);
 // what is known of x when SSOR steps start: nothing, or x = 0 on the active rows

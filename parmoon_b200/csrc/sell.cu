@@ -532,9 +532,8 @@ __global__ void k_csr_to_sell(int nslices, const int *__restrict__ perm, const i
 // the sums kept between the sweeps, zero at first (the first colour's lower and
 // the last colour's upper sums stay 0, the Dirichlet rows' too)
 template <typename T>
-static int alloc_sums(Handle &h, const Level &L, DBuf<T> &sl, DBuf<T> &su, DBuf<T> &base) {
+static int alloc_sums(Handle &h, const Level &L, DBuf<T> &sl, DBuf<T> &su) {
   const size_t n = (size_t)L.sell_nslices * 32;
-  if (!L.blk_col.empty()) PMG_TRY(base.alloc(n));
   if (sl.n == n && su.n == n) return PMG_OK;
   PMG_TRY(sl.alloc(n));
   PMG_TRY(su.alloc(n));
@@ -571,13 +570,11 @@ int sell_values(Handle &h, Level &L) {
   if (f32) {
     PMG_TRY(L.sell_val32.alloc(L.sell_nnz));
     PMG_TRY(L.sell_invd32.alloc((size_t)L.sell_nslices * 32));
-    PMG_TRY(alloc_sums(h, L, L.sell_sl32, L.sell_su32, L.sell_base32));
     val = reinterpret_cast<T *>(L.sell_val32.p);
     invd = reinterpret_cast<T *>(L.sell_invd32.p);
   } else {
     PMG_TRY(L.sell_val64.alloc(L.sell_nnz));
     PMG_TRY(L.sell_invd64.alloc((size_t)L.sell_nslices * 32));
-    PMG_TRY(alloc_sums(h, L, L.sell_sl64, L.sell_su64, L.sell_base64));
     val = reinterpret_cast<T *>(L.sell_val64.p);
     invd = reinterpret_cast<T *>(L.sell_invd64.p);
   }
@@ -587,22 +584,8 @@ int sell_values(Handle &h, Level &L) {
                                                                 L.sell_split ? L.sell_src.p : nullptr, val, invd);
   count_launches(1);
   PMG_CUDA(cudaGetLastError());
-  if (!L.blk_col.empty()) {
-    const int n = (int)(L.blk_meta.n / 4);
-    T *bval;
-    if (f32) {
-      PMG_TRY(L.blk_val32.alloc((size_t)L.blk_chunks * 128));
-      bval = reinterpret_cast<T *>(L.blk_val32.p);
-    } else {
-      PMG_TRY(L.blk_val64.alloc((size_t)L.blk_chunks * 128));
-      bval = reinterpret_cast<T *>(L.blk_val64.p);
-    }
-    k_blk_values<T><<<std::min((n + 7) / 8, h.num_sms * 16), 256, 0, h.stream>>>(
-        n, reinterpret_cast<const int4 *>(L.blk_meta.p), L.sell_ptr.p, L.sell_nlow.p, val, bval);
-    count_launches(1);
-    PMG_CUDA(cudaGetLastError());
-  }
-  if (f32) L.sell_val_fresh32 = true; else L.sell_val_fresh64 = true;
+  if (f32) L.sell_val_fresh32 = true, L.blk_val_fresh32 = false;
+  else L.sell_val_fresh64 = true, L.blk_val_fresh64 = false;
   return PMG_OK;
 }
 template int sell_values<float>(Handle &, Level &);
@@ -1286,6 +1269,33 @@ static bool use_blocks(const Level &L) {
     if (blk_smem<T>(L, (int)p, false) > BLK_SMEM) return false;
   return !L.blk_col.empty();
 }
+
+// What the sweeps need beside the values: the kept sums and, for SSOR steps by
+// blocks, the base vector and the blocks' copy of the entries inside them.  Products
+// need none of it (the FP64 finest matrix of an FP32 V-cycle: at Q2 64^3 0.4 GB and a
+// pass over the matrix per solve).
+template <typename T>
+int sell_sweep_values(Handle &h, Level &L, bool ssor) {
+  const bool f32 = sizeof(T) == 4;
+  PMG_TRY(sell_values<T>(h, L));
+  if (f32) PMG_TRY(alloc_sums(h, L, L.sell_sl32, L.sell_su32));
+  else PMG_TRY(alloc_sums(h, L, L.sell_sl64, L.sell_su64));
+  if (!ssor || !use_blocks<T>(L) || (f32 ? L.blk_val_fresh32 : L.blk_val_fresh64)) return PMG_OK;
+  const size_t rows = (size_t)L.sell_nslices * 32, nval = (size_t)L.blk_chunks * 128;
+  PMG_TRY(f32 ? L.sell_base32.alloc(rows) : L.sell_base64.alloc(rows));
+  PMG_TRY(f32 ? L.blk_val32.alloc(nval) : L.blk_val64.alloc(nval));
+  T *bval = f32 ? reinterpret_cast<T *>(L.blk_val32.p) : reinterpret_cast<T *>(L.blk_val64.p);
+  const int n = (int)(L.blk_meta.n / 4);
+  k_blk_values<T><<<std::min((n + 7) / 8, h.num_sms * 16), 256, 0, h.stream>>>(
+      n, reinterpret_cast<const int4 *>(L.blk_meta.p), L.sell_ptr.p, L.sell_nlow.p, sell_val<T>(L), bval);
+  count_launches(1);
+  PMG_CUDA(cudaGetLastError());
+  if (f32) L.blk_val_fresh32 = true;
+  else L.blk_val_fresh64 = true;
+  return PMG_OK;
+}
+template int sell_sweep_values<float>(Handle &, Level &, bool);
+template int sell_sweep_values<double>(Handle &, Level &, bool);
 
 template <typename T, int MODE>
 static int launch_phase(cudaStream_t st, const Level &L, int p, const T *f, const T *x, int num_sms) {

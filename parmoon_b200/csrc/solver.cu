@@ -712,8 +712,10 @@ static int prepare_levels(Handle &h) {
       const bool jac = h.prm.smoother == PMG_SMOOTHER_JACOBI || (i == 0 && h.prm.coarse_smoother == PMG_COARSE_JACOBI);
       for (int k = 0; k < 3 && slc; k++) PMG_TRY(fp32 ? L.slc32[k].alloc(L.N) : L.slc64[k].alloc(L.N));
       if (jac) PMG_TRY(fp32 ? L.jac32.alloc(L.N) : L.jac64.alloc(L.N));
+      // (the coarsest level is not swept here: dense product or k_coarse_iterate)
+      const bool swept = i > 0 && h.prm.smoother != PMG_SMOOTHER_JACOBI, ssor = h.prm.smoother != PMG_SMOOTHER_SOR;
       if (fp32) {
-        PMG_TRY(sell_values<float>(h, L));
+        PMG_TRY(swept ? sell_sweep_values<float>(h, L, ssor) : sell_values<float>(h, L));
         PMG_TRY(L.x32.alloc(L.N)); PMG_TRY(L.f32.alloc(L.N)); PMG_TRY(L.d32.alloc(L.N));
         if (i > 0 && !L.pval32.p) {
           PMG_TRY(L.pval32.alloc(L.pval.n));
@@ -722,7 +724,7 @@ static int prepare_levels(Handle &h) {
           PMG_TRY(convert_f64_f32(h.stream, L.rval.p, L.rval32.p, L.rval.n));
         }
       } else {
-        PMG_TRY(sell_values<double>(h, L));
+        PMG_TRY(swept ? sell_sweep_values<double>(h, L, ssor) : sell_values<double>(h, L));
       }
     }
     // the outer Krylov method multiplies with the FP64 finest matrix
