@@ -105,6 +105,9 @@ static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std:
     if (S >= nc) break;
     std::vector<int> bound(S + 1);
     for (int p = 0; p <= S; p++) bound[p] = (int)((long)p * nc / S);
+    // (the hops are counted in fixed arrays; and the tables below hold a number per
+    // block and colour, which stays within 64 per row this way)
+    if ((nc + S - 1) / S > BLK_MAX_COLOURS) continue;
     std::vector<int> phase_of(nc + 1, S);
     for (int p = 0; p < S; p++)
       for (int c = bound[p]; c < bound[p + 1]; c++) phase_of[c] = p;
@@ -145,9 +148,6 @@ static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std:
       }
     }
     if (largest > 65535 || largest * sizeof(float) + largest / 32 * BLK_TASK > BLK_SMEM || all > 1.6 * Na) continue;
-    bool narrow = true;  // (the hops are counted in fixed arrays)
-    for (int p = 0; p < S; p++) narrow = narrow && bound[p + 1] - bound[p] <= BLK_MAX_COLOURS;
-    if (!narrow) continue;
     L.blk_col = bound;
     L.blk_n = n;
     return PMG_OK;
