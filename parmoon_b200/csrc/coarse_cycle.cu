@@ -568,7 +568,7 @@ int coarse_cycle_top(Handle &h) {
     const Level &L = h.lv[i];
     bytes += ((size_t)L.N * vb + 15) / 16 * 16;
     if (bytes > CC_SMEM_X || (int)L.sell_group.size() > CC_MAX_GROUPS) break;
-    if (max_rows > 0 && L.N > (L.blk_col.empty() ? max_rows : max_block_rows)) break;
+    if (max_rows > 0 && L.N > (L.blk_on[vb == sizeof(double)] ? max_block_rows : max_rows)) break;
     top = i;
   }
   if (top < 1) return 0;

@@ -188,6 +188,7 @@ struct Level {
   // slots of the block.  blk_tab from blk_tab0[p]: per block its first slice in
   // blk_meta / blk_rows, the first ordinal of every colour, the number of slices
   std::vector<int> blk_col, blk_n, blk_tab0, blk_slots;
+  bool blk_on[2] = {false, false};  // whether SSOR steps run by blocks in FP32 / FP64 (sell.cu, block_gain)
   DBuf<int> blk_tab, blk_meta, blk_rows, sell_in;
   DBuf<unsigned short> sell_loc;
   long blk_chunks = 0;         // chunks of 4 steps of the inside entries

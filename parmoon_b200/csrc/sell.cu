@@ -93,9 +93,10 @@ constexpr int BLK_TASK = 16;  // bytes per task kept beside it
 // Phases and blocks of a level: phase boundaries into L.blk_col (empty: none),
 // block of every active row into blk.  About the cube root of the number of
 // colours as the number of phases first (27 -> 3, 8 -> 2), then finer ones.
-// d_phase, d_parent: N ints of device scratch each.
-static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std::vector<int> &blk, int *d_phase,
-                       int *d_parent) {
+// d_phase, d_parent: N ints of device scratch each.  slices: per phase those of
+// each block.
+static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std::vector<int> &blk,
+                       std::vector<std::vector<int>> &slices, int *d_phase, int *d_parent) {
   const int N = L.N, Na = L.Na, nc = (int)L.rcolor_ptr.size() - 1;
   L.blk_col.clear();
   if (N < BLK_MIN_ROWS || nc < 3) return PMG_OK;
@@ -138,11 +139,13 @@ static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std:
     // a block's slots (rows padded to slices) fit shared memory in FP32 at
     // least, and the padding does not outweigh the rows
     size_t all = 0, largest = 0;
+    slices.assign(S, {});
     for (int p = 0; p < S; p++) {
       const int w = bound[p + 1] - bound[p];
+      slices[p].assign(n[p], 0);
       for (int b = 0; b < n[p]; b++) {
-        size_t slots = 0;
-        for (int c = 0; c < w; c++) slots += ((size_t)rows[p][(size_t)b * w + c] + 31) / 32 * 32;
+        for (int c = 0; c < w; c++) slices[p][b] += (rows[p][(size_t)b * w + c] + 31) / 32;
+        const size_t slots = (size_t)slices[p][b] * 32;
         all += slots;
         largest = std::max(largest, slots);
       }
@@ -153,6 +156,50 @@ static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std:
     return PMG_OK;
   }
   return PMG_OK;
+}
+
+// Whether an SSOR step by blocks is the faster one, per precision: the time of a
+// step's colour launches less that of its products and block sweeps, in us.  A block
+// is swept by one CTA, so what counts is the largest one of a phase, or all of them
+// and a start-up each where there are more than SMs.  The model is fitted to steps
+// on the levels of Q1, Q2, P2 and non-conforming hierarchies of 5 k to 2.1 M rows and
+// on slabs of 33^2 to 201^2 x 9 to 257 nodes (148 SMs): a launch 2.7 us; entries read
+// by the whole GPU 0.4 / 0.2 us per MB (FP32 / FP64; the ones inside blocks are read
+// by a few SMs and are in their terms); a block's slice 0.018 / 0.036 us and 0.009 /
+// 0.016 us for every chunk of four inside entries, per pass; a block beyond the first
+// 148 3.6 us.  It has the sign of the measured difference in 107 of 114 cases; in
+// the others the two are within 11 us of each other.  Measured (us per step, blocks
+// against colours): Q2 64^3 FP32 333 / 366, FP64 568 / 471; Q2 32^3 87 / 163, 117 /
+// 140; Q1 64^3 34 / 60, 51 / 66; Q1 128^3 170 / 186, 304 / 234; Q1 129 x 129 x 9 nodes
+// FP32 86 / 39, 201 x 201 x 9 203 / 51, 65 x 65 x 257 79 / 109; N_Q1 48^3 (1334
+// blocks) 64 / 39.
+static void block_gain(const Level &L, int num_sms, const std::vector<int> &blk, const std::vector<unsigned> &ins,
+                       const std::vector<int> &phase_of_row, const std::vector<std::vector<int>> &slices, int ncol,
+                       double gain[2]) {
+  constexpr double LAUNCH = 2.7, MB[2] = {0.4, 0.2}, SLICE[2] = {0.0184, 0.036}, CHUNK[2] = {0.0093, 0.016},
+                   START = 3.6;
+  const int P = (int)slices.size();
+  std::vector<std::vector<double>> chunks(P);  // per pass
+  for (int p = 0; p < P; p++) chunks[p].assign(slices[p].size(), 0.0);
+  double inside = 0.0;
+  for (int r = 0; r < L.Na; r++) {
+    const int li = ins[r] & 0xffff, ui = ins[r] >> 16;
+    chunks[phase_of_row[r]][blk[r]] += ((li + 3) / 4 + (ui + 3) / 4) / 64.0;
+    inside += li + ui;
+  }
+  for (int t = 0; t < 2; t++) {
+    double sweeps = 0.0;
+    for (int p = 0; p < P; p++) {
+      double most = 0.0, all = -START * num_sms;
+      for (size_t b = 0; b < slices[p].size(); b++) {
+        const double c = SLICE[t] * slices[p][b] + CHUNK[t] * chunks[p][b];
+        most = std::max(most, c);
+        all += c + START;
+      }
+      sweeps += 2.0 * std::max(most, all / num_sms);
+    }
+    gain[t] = LAUNCH * (2 * ncol - 2 - 4 * (P - 1)) + MB[t] * 1e-6 * inside * (t ? 10 : 6) - sweeps;
+  }
 }
 
 // entries of each row in the solve copy: an active row keeps its columns < Na
@@ -289,7 +336,8 @@ int build_sell(Handle &h, Level &L) {
   int *d_colour = h.setup_scratch.p, *d_phase = d_colour + part, *d_nlow = d_phase + part, *d_lptr = d_nlow + part,
       *d_slot = d_lptr + part, *d_rowa = d_slot + part, *d_bad = d_rowa + part;
   std::vector<int> blk;  // block of each active row inside its phase
-  PMG_TRY(find_blocks(h, L, colour, blk, d_rowa, d_nlow));
+  std::vector<std::vector<int>> blk_slices;
+  PMG_TRY(find_blocks(h, L, colour, blk, blk_slices, d_rowa, d_nlow));
   std::vector<int> phase(nc + 1, -1);
   for (size_t p = 0; p + 1 < L.blk_col.size(); p++)
     for (int c = L.blk_col[p]; c < L.blk_col[p + 1]; c++) phase[c] = (int)p;
@@ -319,14 +367,27 @@ int build_sell(Handle &h, Level &L) {
   PMG_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
   PMG_CUDA(cudaStreamSynchronize(h.stream));
   bool split = bad == 0;
-  // (the blocks' tables keep the inside counts in 12 bits)
-  for (int r = 0; r < Na; r++)
-    if ((ins[r] & 0xffff) > 4095 || ins[r] >> 16 > 4095) {
+  L.blk_on[0] = L.blk_on[1] = false;
+  if (!L.blk_col.empty()) {
+    std::vector<int> phase_of_row(Na);
+    bool fits = split;  // (the blocks' tables keep the inside counts in 12 bits)
+    for (int r = 0; r < Na; r++) {
+      phase_of_row[r] = phase[colour[r]];
+      fits = fits && (ins[r] & 0xffff) <= 4095 && ins[r] >> 16 <= 4095;
+    }
+    double gain[2];
+    block_gain(L, h.num_sms, blk, ins, phase_of_row, blk_slices, nc, gain);
+    size_t largest = 0;
+    for (const auto &p : blk_slices)
+      for (int s : p) largest = std::max(largest, (size_t)s);
+    for (int t = 0; t < 2; t++)
+      L.blk_on[t] = fits && gain[t] > 0.0 && largest * ((t ? 8 : 4) * 32 + BLK_TASK) <= BLK_SMEM;
+    if (!L.blk_on[0] && !L.blk_on[1]) {
       L.blk_col.clear();
       std::fill(phase.begin(), phase.end(), -1);
       std::fill(ins.begin(), ins.end(), 0u);
-      break;
     }
+  }
   std::vector<int> dd_row, dd_beg;
   for (int r = 0; r < Na; r++)
     if (rp[r] + alen[r] < rp[r + 1]) {
@@ -341,6 +402,7 @@ int build_sell(Handle &h, Level &L) {
       std::fill(nlow.begin(), nlow.end(), 0);
       std::fill(ins.begin(), ins.end(), 0u);
       L.blk_col.clear();
+      L.blk_on[0] = L.blk_on[1] = false;
     }
     const bool blocks = !L.blk_col.empty();
     // groups: colours of the active rows (block by block), then the Dirichlet rows
@@ -1262,12 +1324,10 @@ static size_t blk_smem(const Level &L, int p, bool turn) {
   return (turn ? 2 : 1) * ((size_t)L.blk_slots[p] * sizeof(T) + (size_t)(L.blk_slots[p] / 32) * BLK_TASK);
 }
 
-// whether the level's sweeps run by blocks in this precision
+// whether the level's SSOR sweeps run by blocks in this precision
 template <typename T>
 static bool use_blocks(const Level &L) {
-  for (size_t p = 0; p + 1 < L.blk_col.size(); p++)
-    if (blk_smem<T>(L, (int)p, false) > BLK_SMEM) return false;
-  return !L.blk_col.empty();
+  return L.blk_on[sizeof(T) == 8];
 }
 
 // What the sweeps need beside the values: the kept sums and, for SSOR steps by
