@@ -98,6 +98,33 @@ struct DBuf {
   ~DBuf() { release(); }
 };
 
+// Several arrays in one allocation (above about 2 MB one takes 0.3 ms whatever its
+// size): add() the sizes, then place() the arrays in the buffer.
+template <typename T>
+struct View {
+  T *p = nullptr;
+  size_t n = 0;
+};
+struct Carve {
+  std::vector<std::pair<void **, size_t>> parts;
+  std::vector<size_t *> counts;
+  size_t bytes = 0;
+  template <typename T>
+  void add(View<T> &v, size_t count) {
+    parts.push_back({reinterpret_cast<void **>(&v.p), bytes});
+    counts.push_back(&v.n);
+    v.n = count;
+    bytes += (count * sizeof(T) + 255) / 256 * 256;
+  }
+  int place(DBuf<unsigned char> &buf) {
+    const int rc = buf.alloc(bytes);
+    for (auto &q : parts) *q.first = rc == PMG_OK ? buf.p + q.second : nullptr;
+    if (rc != PMG_OK)
+      for (size_t *n : counts) *n = 0;
+    return rc;
+  }
+};
+
 // element descriptors
 struct ElemInfo {
   int nloc, nvert, quad_default;
@@ -164,23 +191,25 @@ struct Level {
   int sell_nslices = 0;
   long sell_nnz = 0;
   std::vector<int> sell_group;  // slice range of each colour group (+ Dirichlet group)
-  DBuf<int> sell_perm, sell_ptr, sell_col;
+  DBuf<unsigned char> sell_mem;  // tables and columns of the copy
+  View<int> sell_perm, sell_ptr, sell_col;
   // solve copy of an active row = its columns < Na (a prefix: columns are
   // sorted); the Dirichlet columns are applied separately (dd_row / dd_beg)
-  DBuf<short> sell_c16;          // column - the lane's row, for slices whose deltas fit 16 bits
-  DBuf<unsigned char> sell_wide; // 1: the slice keeps 32-bit columns (sell_col)
-  DBuf<int> sell_alen;           // entries of each row in the solve copy
-  DBuf<int> dd_row, dd_beg;      // active rows with Dirichlet columns, first such CSR position
+  View<short> sell_c16;          // column - the lane's row, for slices whose deltas fit 16 bits
+  View<unsigned char> sell_wide; // 1: the slice keeps 32-bit columns (sell_col)
+  View<int> sell_alen;           // entries of each row in the solve copy
+  View<int> dd_row, dd_beg;      // active rows with Dirichlet columns, first such CSR position
   int n_dd = 0;
   // the rows' entries split by colour: steps [0, nlow) of a slice hold the
   // columns of lower colours, step nlow the diagonal, the rest the higher
   // ones; sell_src: an entry's position in its CSR row (SELL_NO_SRC: padding)
   bool sell_split = false;
   bool sell_coupled = false;  // two rows of one colour are coupled (then not split either)
-  DBuf<int> sell_nlow;
-  DBuf<unsigned short> sell_src;
-  DBuf<float> sell_sl32, sell_su32;  // sums over the lower / higher colours kept between sweeps
-  DBuf<double> sell_sl64, sell_su64;
+  View<int> sell_nlow;
+  View<unsigned short> sell_src;
+  DBuf<unsigned char> sums_mem32, sums_mem64;
+  View<float> sell_sl32, sell_su32;  // sums over the lower / higher colours kept between sweeps
+  View<double> sell_sl64, sell_su64;
   // phases and blocks of the sweeps (sell.cu, find_blocks): phase p holds the
   // colours [blk_col[p], blk_col[p + 1]); its rows fall into blk_n[p] blocks
   // that are not coupled inside the phase.  sell_in: a slice's steps in its own
@@ -189,17 +218,19 @@ struct Level {
   // blk_meta / blk_rows, the first ordinal of every colour, the number of slices
   std::vector<int> blk_col, blk_n, blk_tab0, blk_slots;
   bool blk_on[2] = {false, false};  // whether SSOR steps run by blocks in FP32 / FP64 (sell.cu, block_gain)
-  DBuf<int> blk_tab, blk_meta, blk_rows, sell_in;
-  DBuf<unsigned short> sell_loc;
+  View<int> blk_tab, blk_meta, blk_rows, sell_in;
+  View<unsigned short> sell_loc;
   long blk_chunks = 0;         // chunks of 4 steps of the inside entries
-  DBuf<float> blk_val32;       // their values in that layout
-  DBuf<double> blk_val64;
+  DBuf<unsigned char> blk_mem32, blk_mem64;
+  View<float> blk_val32;       // their values in that layout
+  View<double> blk_val64;
   bool blk_val_fresh32 = false, blk_val_fresh64 = false;  // hold the solve copy's present values
-  DBuf<float> sell_base32;   // f minus the sums from outside the block (slice order)
-  DBuf<double> sell_base64;
+  View<float> sell_base32;   // f minus the sums from outside the block (slice order)
+  View<double> sell_base64;
   long sell_nnz_narrow = 0, sell_nnz_wide = 0;  // stored entries with 16-bit / 32-bit columns
-  DBuf<float> sell_val32, sell_invd32;
-  DBuf<double> sell_val64, sell_invd64;
+  DBuf<unsigned char> val_mem32, val_mem64;
+  View<float> sell_val32, sell_invd32;
+  View<double> sell_val64, sell_invd64;
 };
 
 // Activations and gradients of the stencil network: node-major BF16 (32
@@ -248,13 +279,17 @@ struct Handle {
   int num_sms = 148;
   // coarsest-level dense inverse (FP64)
   // active block: work array, pivot rows, inverse before and after its Newton step; reduced rhs
-  DBuf<double> coarse_lu, coarse_w, coarse_x, coarse_inv, coarse_t;
-  DBuf<int> coarse_piv, coarse_perm;  // pivot row of each column, column of each row
+  DBuf<unsigned char> coarse_mem;
+  View<double> coarse_lu, coarse_w, coarse_x, coarse_inv;
+  DBuf<double> coarse_t;
+  View<int> coarse_piv, coarse_perm;  // pivot row of each column, column of each row
   DBuf<int> coarse_cptr;  // colour pointers of the coarsest level's rows (iterative coarse solve)
   bool coarse_ready = false;
   // FGMRES workspace
   int krylov_n = 0, krylov_restart = 0;
-  DBuf<double> V, Z, w, sol, rhs, H, scal;
+  DBuf<unsigned char> krylov_mem;
+  View<double> V, Z, H;
+  DBuf<double> w, sol, rhs, scal;
   DBuf<double> red_partial;
   DBuf<double> slc_part;  // step-length control: block partials of (d0, y), (y, y) and alpha
   DBuf<unsigned int> red_counter;

@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 
 namespace pmg {
 
@@ -61,12 +62,12 @@ __device__ __forceinline__ int cc_find(int *parent, int i) {
 // union of the two ends of every entry inside a phase (a root only ever gets a
 // smaller parent, so the trees have no cycles and every loop ends)
 __global__ void k_cc_unite(int Na, const int *__restrict__ rp, const int *__restrict__ kc,
-                           const int *__restrict__ phase, int *parent) {
+                           const int *__restrict__ colour, const int *__restrict__ phase, int *parent) {
   const int lane = threadIdx.x & 31;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < Na; r += (gridDim.x * blockDim.x) >> 5)
     for (int k = rp[r] + lane; k < rp[r + 1]; k += 32) {
       const int c = kc[k];
-      if (c >= Na || c == r || phase[c] != phase[r]) continue;
+      if (c >= Na || c == r || phase[colour[c]] != phase[colour[r]]) continue;
       int a = cc_find(parent, r), b = cc_find(parent, c);
       while (a != b) {
         if (a < b) { const int t = a; a = b; b = t; }
@@ -77,9 +78,14 @@ __global__ void k_cc_unite(int Na, const int *__restrict__ rp, const int *__rest
       }
     }
 }
-__global__ void k_cc_flatten(int n, int *parent) {
+// (and the number of components of every phase)
+__global__ void k_cc_flatten(int n, const int *__restrict__ colour, const int *__restrict__ phase, int *parent,
+                             int *count) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) parent[i] = cc_find(parent, i);
+  if (i >= n) return;
+  const int root = cc_find(parent, i);
+  parent[i] = root;
+  if (root == i) atomicAdd(count + phase[colour[i]], 1);
 }
 
 // Smaller levels run in the coarse cycle's cluster launch (coarse_cycle.cu has the
@@ -93,15 +99,16 @@ constexpr int BLK_TASK = 16;  // bytes per task kept beside it
 // Phases and blocks of a level: phase boundaries into L.blk_col (empty: none),
 // block of every active row into blk.  About the cube root of the number of
 // colours as the number of phases first (27 -> 3, 8 -> 2), then finer ones.
-// d_phase, d_parent: N ints of device scratch each.  slices: per phase those of
-// each block.
+// d_colour: the colours on the device; d_phase, d_parent, d_count: device scratch of
+// N + colours ints each.  slices: per phase those of each block.
 static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std::vector<int> &blk,
-                       std::vector<std::vector<int>> &slices, int *d_phase, int *d_parent) {
+                       std::vector<std::vector<int>> &slices, const int *d_colour, int *d_phase, int *d_parent,
+                       int *d_count) {
   const int N = L.N, Na = L.Na, nc = (int)L.rcolor_ptr.size() - 1;
   L.blk_col.clear();
   if (N < BLK_MIN_ROWS || nc < 3) return PMG_OK;
   const int s0 = std::max(2, (int)(cbrt((double)nc) + 0.5));
-  std::vector<int> phase(N), label(Na);
+  std::vector<int> label;
   for (int S : {s0, s0 + 1, s0 * s0}) {
     if (S >= nc) break;
     std::vector<int> bound(S + 1);
@@ -112,27 +119,31 @@ static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std:
     std::vector<int> phase_of(nc + 1, S);
     for (int p = 0; p < S; p++)
       for (int c = bound[p]; c < bound[p + 1]; c++) phase_of[c] = p;
-    for (int r = 0; r < N; r++) phase[r] = phase_of[colour[r]];
-    PMG_CUDA(cudaMemcpyAsync(d_phase, phase.data(), sizeof(int) * N, cudaMemcpyHostToDevice, h.stream));
+    PMG_CUDA(cudaMemcpyAsync(d_phase, phase_of.data(), sizeof(int) * (nc + 1), cudaMemcpyHostToDevice, h.stream));
+    PMG_CUDA(cudaMemsetAsync(d_count, 0, sizeof(int) * S, h.stream));
     k_cc_init<<<(Na + 255) / 256, 256, 0, h.stream>>>(Na, d_parent);
-    k_cc_unite<<<h.num_sms * 8, 256, 0, h.stream>>>(Na, L.rowptr.p, L.kcol.p, d_phase, d_parent);
-    k_cc_flatten<<<(Na + 255) / 256, 256, 0, h.stream>>>(Na, d_parent);
+    k_cc_unite<<<h.num_sms * 8, 256, 0, h.stream>>>(Na, L.rowptr.p, L.kcol.p, d_colour, d_phase, d_parent);
+    k_cc_flatten<<<(Na + 255) / 256, 256, 0, h.stream>>>(Na, d_colour, d_phase, d_parent, d_count);
     count_launches(3);
     PMG_CUDA(cudaGetLastError());
-    PMG_CUDA(cudaMemcpyAsync(label.data(), d_parent, sizeof(int) * Na, cudaMemcpyDeviceToHost, h.stream));
-    PMG_CUDA(cudaStreamSynchronize(h.stream));
-    // number the blocks of each phase by their first rows; rows per block and colour
     std::vector<int> n(S, 0);
-    blk.assign(Na, -1);
-    for (int r = 0; r < Na; r++)
-      if (label[r] == r) blk[r] = n[phase[r]]++;
+    PMG_CUDA(cudaMemcpyAsync(n.data(), d_count, sizeof(int) * S, cudaMemcpyDeviceToHost, h.stream));
+    PMG_CUDA(cudaStreamSynchronize(h.stream));
     bool ok = true;
     for (int p = 0; p < S; p++) ok = ok && n[p] >= 4 && n[p] <= 65535;
     if (!ok) continue;
+    label.resize(Na);
+    PMG_CUDA(cudaMemcpyAsync(label.data(), d_parent, sizeof(int) * Na, cudaMemcpyDeviceToHost, h.stream));
+    PMG_CUDA(cudaStreamSynchronize(h.stream));
+    // number the blocks of each phase by their first rows; rows per block and colour
+    std::fill(n.begin(), n.end(), 0);
+    blk.assign(Na, -1);
+    for (int r = 0; r < Na; r++)
+      if (label[r] == r) blk[r] = n[phase_of[colour[r]]]++;
     std::vector<std::vector<int>> rows(S);
     for (int p = 0; p < S; p++) rows[p].assign((size_t)n[p] * (bound[p + 1] - bound[p]), 0);
     for (int r = 0; r < Na; r++) {
-      const int p = phase[r];
+      const int p = phase_of[colour[r]];
       blk[r] = blk[label[r]];
       rows[p][(size_t)blk[r] * (bound[p + 1] - bound[p]) + colour[r] - bound[p]]++;
     }
@@ -332,12 +343,19 @@ int build_sell(Handle &h, Level &L) {
   // (an allocation can take longer than all the kernels here)
   // (a slice holds a row, so there are at most N; even parts keep 8-byte alignment)
   const size_t part = ((size_t)N + nc + 64) / 2 * 2;
-  PMG_TRY(h.setup_scratch.reserve(7 * part));
+  size_t most = part;  // (the largest level's at once, not level by level)
+  for (const Level &o : h.lv) most = std::max(most, ((size_t)o.N + o.rcolor_ptr.size() + 64) / 2 * 2);
+  PMG_TRY(h.setup_scratch.reserve(8 * most));
   int *d_colour = h.setup_scratch.p, *d_phase = d_colour + part, *d_nlow = d_phase + part, *d_lptr = d_nlow + part,
-      *d_slot = d_lptr + part, *d_rowa = d_slot + part, *d_bad = d_rowa + part;
+      *d_slot = d_lptr + part, *d_rowa = d_slot + part, *d_alen = d_rowa + part, *d_bad = d_alen + part;
   std::vector<int> blk;  // block of each active row inside its phase
   std::vector<std::vector<int>> blk_slices;
-  PMG_TRY(find_blocks(h, L, colour, blk, blk_slices, d_rowa, d_nlow));
+  auto put = [&](int *d, const std::vector<int> &v) {
+    return v.empty() ? cudaSuccess
+                     : cudaMemcpyAsync(d, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, h.stream);
+  };
+  PMG_CUDA(put(d_colour, colour));
+  PMG_TRY(find_blocks(h, L, colour, blk, blk_slices, d_colour, d_phase, d_nlow, d_rowa));
   std::vector<int> phase(nc + 1, -1);
   for (size_t p = 0; p + 1 < L.blk_col.size(); p++)
     for (int c = L.blk_col[p]; c < L.blk_col[p + 1]; c++) phase[c] = (int)p;
@@ -349,19 +367,13 @@ int build_sell(Handle &h, Level &L) {
   std::vector<unsigned> ins(N);
   unsigned *d_ins = reinterpret_cast<unsigned *>(d_rowa);
   int bad = 0;
-  auto put = [&](int *d, const std::vector<int> &v) {
-    return v.empty() ? cudaSuccess
-                     : cudaMemcpyAsync(d, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, h.stream);
-  };
-  PMG_CUDA(put(d_colour, colour));
   PMG_CUDA(put(d_phase, phase));
-  PMG_TRY(L.sell_alen.alloc(N));
   PMG_CUDA(cudaMemsetAsync(d_bad, 0, 8 * sizeof(int), h.stream));
-  k_row_counts<<<h.num_sms * 8, 256, 0, h.stream>>>(N, Na, L.rowptr.p, L.kcol.p, d_colour, d_phase, L.sell_alen.p,
-                                                    d_nlow, d_ins, d_bad);
+  k_row_counts<<<h.num_sms * 8, 256, 0, h.stream>>>(N, Na, L.rowptr.p, L.kcol.p, d_colour, d_phase, d_alen, d_nlow,
+                                                    d_ins, d_bad);
   count_launches(1);
   PMG_CUDA(cudaGetLastError());
-  PMG_CUDA(cudaMemcpyAsync(alen.data(), L.sell_alen.p, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
+  PMG_CUDA(cudaMemcpyAsync(alen.data(), d_alen, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
   PMG_CUDA(cudaMemcpyAsync(nlow.data(), d_nlow, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
   PMG_CUDA(cudaMemcpyAsync(ins.data(), d_ins, sizeof(int) * N, cudaMemcpyDeviceToHost, h.stream));
   PMG_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
@@ -413,17 +425,30 @@ int build_sell(Handle &h, Level &L) {
       if (g < nc) rows.assign(L.h_row_list.begin() + L.rcolor_ptr[g], L.h_row_list.begin() + L.rcolor_ptr[g + 1]);
       else for (int r = Na; r < N; r++) rows.push_back(r);
       const bool by_block = blocks && g < nc;
-      std::sort(rows.begin(), rows.end(), [&](int a, int b) {
-        if (by_block && blk[a] != blk[b]) return blk[a] < blk[b];
-        if (alen[a] != alen[b]) return alen[a] > alen[b];
-        if (nlow[a] != nlow[b]) return nlow[a] > nlow[b];
-        if (ins[a] != ins[b]) return ins[a] > ins[b];
-        return a < b;
-      });
+      // by block, then longest row, longest lower part, most inside entries first (the
+      // keys side by side: a comparator that looks them up takes three times as long)
+      struct Key {
+        int blk, len, low;
+        unsigned ins;
+        int row;
+      };
+      std::vector<Key> key(rows.size());
       for (size_t k = 0; k < rows.size(); k++) {
-        if (by_block && k > 0 && blk[rows[k]] != blk[rows[k - 1]])
+        const int r = rows[k];
+        key[k] = {by_block ? blk[r] : 0, alen[r], nlow[r], r < Na ? ins[r] : 0u, r};
+      }
+      std::sort(key.begin(), key.end(), [](const Key &a, const Key &b) {
+        if (a.blk != b.blk) return a.blk < b.blk;
+        if (a.len != b.len) return a.len > b.len;
+        if (a.low != b.low) return a.low > b.low;
+        if (a.ins != b.ins) return a.ins > b.ins;
+        return a.row < b.row;
+      });
+      out.reserve(rows.size() + 32);
+      for (size_t k = 0; k < key.size(); k++) {
+        if (k > 0 && key[k].blk != key[k - 1].blk)
           while (out.size() % 32) out.push_back(-1);
-        out.push_back(rows[k]);
+        out.push_back(key[k].row);
       }
       while (out.size() % 32) out.push_back(-1);
     }
@@ -508,23 +533,39 @@ int build_sell(Handle &h, Level &L) {
       L.blk_slots.push_back(slots);
     }
   }
-  PMG_TRY(L.sell_perm.upload(perm.data(), perm.size(), h.stream));
-  PMG_TRY(L.sell_ptr.upload(sptr.data(), sptr.size(), h.stream));
-  PMG_TRY(L.sell_nlow.upload(snlow.data(), snlow.size(), h.stream));
-  PMG_TRY(L.sell_in.upload(sin.data(), sin.size(), h.stream));
-  PMG_TRY(L.blk_tab.upload(tab.data(), tab.size(), h.stream));
-  PMG_TRY(L.blk_meta.upload(meta.data(), meta.size(), h.stream));
-  PMG_TRY(L.blk_rows.upload(brows.data(), brows.size(), h.stream));
+  // one allocation; its first part comes from the host in one copy
+  L.n_dd = (int)dd_row.size();
+  Carve parts;
+  parts.add(L.sell_perm, perm.size());
+  parts.add(L.sell_ptr, sptr.size());
+  parts.add(L.sell_nlow, snlow.size());
+  parts.add(L.sell_in, sin.size());
+  parts.add(L.blk_tab, tab.size());
+  parts.add(L.blk_meta, meta.size());
+  parts.add(L.blk_rows, brows.size());
+  parts.add(L.dd_row, dd_row.size());
+  parts.add(L.dd_beg, dd_beg.size());
+  std::vector<unsigned char> host(parts.bytes);
+  {
+    const std::vector<int> *from[] = {&perm, &sptr, &snlow, &sin, &tab, &meta, &brows, &dd_row, &dd_beg};
+    for (size_t k = 0; k < parts.parts.size(); k++)
+      if (!from[k]->empty()) memcpy(&host[parts.parts[k].second], from[k]->data(), from[k]->size() * sizeof(int));
+  }
+  parts.add(L.sell_alen, N);
+  parts.add(L.sell_wide, nslices);
+  parts.add(L.sell_col, total);
+  parts.add(L.sell_c16, total);
+  parts.add(L.sell_src, split ? total : 0);
+  parts.add(L.sell_loc, (size_t)total_in * 128);
+  PMG_TRY(parts.place(L.sell_mem));
+  if (!host.empty())
+    PMG_CUDA(cudaMemcpyAsync(L.sell_mem.p, host.data(), host.size(), cudaMemcpyHostToDevice, h.stream));
+  PMG_CUDA(cudaMemcpyAsync(L.sell_alen.p, d_alen, sizeof(int) * N, cudaMemcpyDeviceToDevice, h.stream));
   // the slices' columns, filled on the device
   unsigned long long *d_nnz = reinterpret_cast<unsigned long long *>(d_bad + 2), nnz[2] = {0, 0};
   PMG_CUDA(put(d_lptr, lptr));
   PMG_CUDA(put(d_slot, slot));
   PMG_CUDA(put(d_phase, phase));
-  PMG_TRY(L.sell_col.alloc(total));
-  PMG_TRY(L.sell_c16.alloc(total));
-  PMG_TRY(L.sell_src.alloc(split ? total : 0));
-  PMG_TRY(L.sell_wide.alloc(nslices));
-  PMG_TRY(L.sell_loc.alloc((size_t)total_in * 128));
   if (nslices > 0) {
     k_sell_fill<<<std::min((nslices + 7) / 8, h.num_sms * 16), 256, 0, h.stream>>>(
         nslices, Na, split, L.sell_perm.p, L.sell_ptr.p, L.sell_nlow.p, L.sell_in.p, d_lptr, L.rowptr.p, L.kcol.p,
@@ -534,15 +575,12 @@ int build_sell(Handle &h, Level &L) {
     PMG_CUDA(cudaGetLastError());
   }
   PMG_CUDA(cudaMemcpyAsync(nnz, d_nnz, sizeof(nnz), cudaMemcpyDeviceToHost, h.stream));
-  L.n_dd = (int)dd_row.size();
-  PMG_TRY(L.dd_row.upload(dd_row.data(), dd_row.size(), h.stream));
-  PMG_TRY(L.dd_beg.upload(dd_beg.data(), dd_beg.size(), h.stream));
   PMG_CUDA(cudaStreamSynchronize(h.stream));
-  // their zeros (see alloc_sums) belong to the old layout
-  L.sell_sl32.release();
-  L.sell_su32.release();
-  L.sell_sl64.release();
-  L.sell_su64.release();
+  // these belong to the old layout
+  L.sums_mem32.release();
+  L.sums_mem64.release();
+  L.blk_mem32.release();
+  L.blk_mem64.release();
   L.blk_chunks = total_in;
   L.sell_group = group_slice;
   L.sell_nslices = nslices;
@@ -594,13 +632,14 @@ __global__ void k_csr_to_sell(int nslices, const int *__restrict__ perm, const i
 // the sums kept between the sweeps, zero at first (the first colour's lower and
 // the last colour's upper sums stay 0, the Dirichlet rows' too)
 template <typename T>
-static int alloc_sums(Handle &h, const Level &L, DBuf<T> &sl, DBuf<T> &su) {
+static int alloc_sums(Handle &h, const Level &L, DBuf<unsigned char> &mem, View<T> &sl, View<T> &su) {
+  if (mem.p) return PMG_OK;  // (released with the layout)
   const size_t n = (size_t)L.sell_nslices * 32;
-  if (sl.n == n && su.n == n) return PMG_OK;
-  PMG_TRY(sl.alloc(n));
-  PMG_TRY(su.alloc(n));
-  PMG_CUDA(cudaMemsetAsync(sl.p, 0, n * sizeof(T), h.stream));
-  PMG_CUDA(cudaMemsetAsync(su.p, 0, n * sizeof(T), h.stream));
+  Carve parts;
+  parts.add(sl, n);
+  parts.add(su, n);
+  PMG_TRY(parts.place(mem));
+  PMG_CUDA(cudaMemsetAsync(mem.p, 0, mem.n, h.stream));
   return PMG_OK;
 }
 
@@ -630,13 +669,17 @@ int sell_values(Handle &h, Level &L) {
   PMG_TRY(build_sell(h, L));
   T *val, *invd;
   if (f32) {
-    PMG_TRY(L.sell_val32.alloc(L.sell_nnz));
-    PMG_TRY(L.sell_invd32.alloc((size_t)L.sell_nslices * 32));
+    Carve parts;
+    parts.add(L.sell_val32, L.sell_nnz);
+    parts.add(L.sell_invd32, (size_t)L.sell_nslices * 32);
+    PMG_TRY(parts.place(L.val_mem32));
     val = reinterpret_cast<T *>(L.sell_val32.p);
     invd = reinterpret_cast<T *>(L.sell_invd32.p);
   } else {
-    PMG_TRY(L.sell_val64.alloc(L.sell_nnz));
-    PMG_TRY(L.sell_invd64.alloc((size_t)L.sell_nslices * 32));
+    Carve parts;
+    parts.add(L.sell_val64, L.sell_nnz);
+    parts.add(L.sell_invd64, (size_t)L.sell_nslices * 32);
+    PMG_TRY(parts.place(L.val_mem64));
     val = reinterpret_cast<T *>(L.sell_val64.p);
     invd = reinterpret_cast<T *>(L.sell_invd64.p);
   }
@@ -1338,12 +1381,14 @@ template <typename T>
 int sell_sweep_values(Handle &h, Level &L, bool ssor) {
   const bool f32 = sizeof(T) == 4;
   PMG_TRY(sell_values<T>(h, L));
-  if (f32) PMG_TRY(alloc_sums(h, L, L.sell_sl32, L.sell_su32));
-  else PMG_TRY(alloc_sums(h, L, L.sell_sl64, L.sell_su64));
+  if (f32) PMG_TRY(alloc_sums(h, L, L.sums_mem32, L.sell_sl32, L.sell_su32));
+  else PMG_TRY(alloc_sums(h, L, L.sums_mem64, L.sell_sl64, L.sell_su64));
   if (!ssor || !use_blocks<T>(L) || (f32 ? L.blk_val_fresh32 : L.blk_val_fresh64)) return PMG_OK;
   const size_t rows = (size_t)L.sell_nslices * 32, nval = (size_t)L.blk_chunks * 128;
-  PMG_TRY(f32 ? L.sell_base32.alloc(rows) : L.sell_base64.alloc(rows));
-  PMG_TRY(f32 ? L.blk_val32.alloc(nval) : L.blk_val64.alloc(nval));
+  Carve parts;
+  if (f32) parts.add(L.sell_base32, rows), parts.add(L.blk_val32, nval);
+  else parts.add(L.sell_base64, rows), parts.add(L.blk_val64, nval);
+  PMG_TRY(parts.place(f32 ? L.blk_mem32 : L.blk_mem64));
   T *bval = f32 ? reinterpret_cast<T *>(L.blk_val32.p) : reinterpret_cast<T *>(L.blk_val64.p);
   const int n = (int)(L.blk_meta.n / 4);
   k_blk_values<T><<<std::min((n + 7) / 8, h.num_sms * 16), 256, 0, h.stream>>>(

@@ -339,12 +339,14 @@ static int coarse_factor_launch(Handle &h, cudaStream_t s) {
     h.h_coarse_flags[0] = 0;
     return PMG_OK;
   }
-  PMG_TRY(h.coarse_lu.alloc((size_t)n * n));
-  PMG_TRY(h.coarse_x.alloc((size_t)n * n));
-  PMG_TRY(h.coarse_inv.alloc((size_t)n * n));
-  PMG_TRY(h.coarse_w.alloc((size_t)GJ_NB * n));
-  PMG_TRY(h.coarse_piv.alloc(n));
-  PMG_TRY(h.coarse_perm.alloc(n));
+  Carve parts;
+  parts.add(h.coarse_lu, (size_t)n * n);
+  parts.add(h.coarse_x, (size_t)n * n);
+  parts.add(h.coarse_inv, (size_t)n * n);
+  parts.add(h.coarse_w, (size_t)GJ_NB * n);
+  parts.add(h.coarse_piv, n);
+  parts.add(h.coarse_perm, n);
+  PMG_TRY(parts.place(h.coarse_mem));
   PMG_CUDA(cudaMemsetAsync(h.coarse_flags.p, 0, sizeof(int) * 4, s));
   double *M = h.coarse_lu.p;
   k_csr_to_dense_active<<<n, 256, 0, s>>>(n, L.rowptr.p, L.kcol.p, L.A.p, M);
@@ -838,6 +840,22 @@ static void givens(double &dx, double &dy, double &cs, double &sn) {
   else { double t = dy / dx; cs = 1.0 / sqrt(1.0 + t * t); sn = t * cs; }
 }
 
+// the Krylov vectors for N rows and m columns
+static int krylov_alloc(Handle &h, size_t N, int m) {
+  Carve parts;
+  parts.add(h.V, N * (m + 1));
+  parts.add(h.Z, N * m);
+  parts.add(h.H, (size_t)(m + 1) * (m + 1) + 64);
+  h.krylov_n = h.krylov_restart = 0;
+  PMG_TRY(parts.place(h.krylov_mem));
+  PMG_TRY(h.w.alloc(N));
+  PMG_TRY(h.sol.alloc(N));
+  PMG_TRY(h.rhs.alloc(N));
+  h.krylov_n = (int)N;
+  h.krylov_restart = m;
+  return PMG_OK;
+}
+
 int solve(Handle &h, double *sol_host, const double *rhs_host, pmg_solve_stats *st) {
   if (h.lv.empty()) { set_error("solve: no levels"); return PMG_ERR_STATE; }
   // the solve's device time covers everything below: per-solve set-up (SELL
@@ -852,14 +870,7 @@ int solve(Handle &h, double *sol_host, const double *rhs_host, pmg_solve_stats *
   const int m = h.prm.restart > 0 ? h.prm.restart : 10;
   if (m > 60) { set_error("solve: restart must be <= 60"); return PMG_ERR_ARG; }
   if (h.krylov_n != (int)N || h.krylov_restart != m) {
-    PMG_TRY(h.V.alloc(N * (m + 1)));
-    PMG_TRY(h.Z.alloc(N * m));
-    PMG_TRY(h.w.alloc(N));
-    PMG_TRY(h.sol.alloc(N));
-    PMG_TRY(h.rhs.alloc(N));
-    PMG_TRY(h.H.alloc((size_t)(m + 1) * (m + 1) + 64));
-    h.krylov_n = (int)N;
-    h.krylov_restart = m;
+    PMG_TRY(krylov_alloc(h, N, m));
   }
   cudaStream_t s = h.stream;
   if (rhs_host) PMG_CUDA(cudaMemcpyAsync(h.rhs.p, rhs_host, sizeof(double) * N, cudaMemcpyHostToDevice, s));
@@ -1099,14 +1110,7 @@ int solve_dd(Handle &h, const pmg_comm *comm, double *sol_host, const double *rh
   const size_t N = F.N;
   const int m = h.prm.restart;
   if (h.krylov_n != (int)N || h.krylov_restart != m) {
-    PMG_TRY(h.V.alloc(N * (m + 1)));
-    PMG_TRY(h.Z.alloc(N * m));
-    PMG_TRY(h.w.alloc(N));
-    PMG_TRY(h.sol.alloc(N));
-    PMG_TRY(h.rhs.alloc(N));
-    PMG_TRY(h.H.alloc((size_t)(m + 1) * (m + 1) + 64));
-    h.krylov_n = (int)N;
-    h.krylov_restart = m;
+    PMG_TRY(krylov_alloc(h, N, m));
   }
   cudaStream_t s = h.stream;
   if (rhs_host) PMG_CUDA(cudaMemcpyAsync(h.rhs.p, rhs_host, sizeof(double) * N, cudaMemcpyHostToDevice, s));
