@@ -527,7 +527,7 @@ static int cluster_ctas() {
 // the highest level that, with every level below it, fits the cluster launch
 // (0: none -- the level-by-level path runs).  By default an 8-CTA cluster takes
 // the levels of at most CC_ROWS rows, and of at most CC_BLOCK_ROWS where the
-// level's sweeps can run by blocks (sell.cu).  Measured: a level of 4,913 rows
+// level's SSOR steps run by blocks (sell.cu).  Measured: a level of 4,913 rows
 // (Q2 8^3) in the cluster 0.29 ms per V-cycle more than by blocks (FP64 V-cycle
 // of the 32^3 Q2 hierarchy 1.25 against 0.95 ms; Q1 32^3 Poisson solve 2.99
 // against 1.99 ms), one of 729 rows 0.02 ms less; without blocks the colour
@@ -538,7 +538,7 @@ static int cluster_ctas() {
 // levels of at most 8192 rows on an 8-CTA cluster whether or not they have
 // blocks, "1" the levels of at most CC_ONE_CTA_ROWS rows on one CTA, "16" (2, 4,
 // 8) every level whose iterates fit CC_SMEM_X on a cluster of that size, "0" none.
-constexpr int CC_ROWS = 8192, CC_BLOCK_ROWS = 2000;
+constexpr int CC_ROWS = 8192;  // (CC_BLOCK_ROWS: pmg_internal.h)
 constexpr int CC_ONE_CTA_ROWS = 8192;
 
 int coarse_cycle_top(Handle &h) {

@@ -132,6 +132,10 @@ struct ElemInfo {
 ElemInfo elem_info(int elem_type);
 
 constexpr int SELL_NO_SRC = 65535;
+// levels of at most this many rows run in the coarse cycle's cluster launch whether
+// or not blocks could be found (coarse_cycle.cu has the measurements), so none are
+// looked for there
+constexpr int CC_BLOCK_ROWS = 2000;
 
 // one multigrid level
 struct Level {
@@ -363,8 +367,9 @@ int prolongate_add(cudaStream_t s, const Level &Lf, const T *pval, const T *xc, 
 int convert_f64_f32(cudaStream_t s, const double *a, float *b, size_t n);
 int copy_dirichlet(cudaStream_t s, int Na, int N, const double *f, double *x);
 int dot(Handle &h, const double *a, const double *b, size_t n, double *result_dev);
-// w -= (*hk_dev) vk, then *h_next = w . u (u = w: the squared norm)
+// column i of the Arnoldi process (sparse.cu)
 int arnoldi_column(Handle &h, size_t n, int i, double *V, double *w, double *hc, double *hc_host);
+// w -= (*hk_dev) vk, then *h_next = w . u (u = w: the squared norm)
 int mgs_step(Handle &h, size_t n, const double *hk_dev, const double *vk, const double *u, double *w, double *h_next);
 int scale_by_inv_sqrt(cudaStream_t s, size_t n, const double *nrm2_dev, const double *x, double *y);
 int fill(cudaStream_t s, double *x, double v, size_t n);

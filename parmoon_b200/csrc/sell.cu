@@ -88,9 +88,6 @@ __global__ void k_cc_flatten(int n, const int *__restrict__ colour, const int *_
   if (root == i) atomicAdd(count + phase[colour[i]], 1);
 }
 
-// Smaller levels run in the coarse cycle's cluster launch (coarse_cycle.cu has the
-// measurements), or are the coarsest one.
-constexpr int BLK_MIN_ROWS = 2001;
 // a block's iterate sits in shared memory, addressed by 16-bit slots
 constexpr size_t BLK_SMEM = 224 * 1024;
 constexpr int BLK_MAX_COLOURS = 64;
@@ -106,7 +103,7 @@ static int find_blocks(Handle &h, Level &L, const std::vector<int> &colour, std:
                        int *d_count) {
   const int N = L.N, Na = L.Na, nc = (int)L.rcolor_ptr.size() - 1;
   L.blk_col.clear();
-  if (N < BLK_MIN_ROWS || nc < 3) return PMG_OK;
+  if (N <= CC_BLOCK_ROWS || nc < 3) return PMG_OK;
   const int s0 = std::max(2, (int)(cbrt((double)nc) + 0.5));
   std::vector<int> label;
   for (int S : {s0, s0 + 1, s0 * s0}) {
