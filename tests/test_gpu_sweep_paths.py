@@ -158,3 +158,18 @@ def test_turn_in_two_launches(pmg, oracle, side, prec):
                           dict(N=n, Na=n, rp=rp, kc=kc, a=a, colors=colors, n_colors=64, P=P)], v, coarse_direct=True)
     err = np.max(np.abs(zd.cpu().numpy() - zo)) / np.max(np.abs(zo))
     assert err < (1e-4 if prec else 1e-10), err
+
+
+@pytest.mark.parametrize("first", [0, 1])
+def test_layout_follows_the_precision_in_use(pmg, first):
+    """65 x 65 x 13 nodes, 8 colours: blocks are the faster way in FP32 only.  A level first used in
+    FP64 is not laid out by blocks at all, one first used in FP32 is, and FP64 sweeps go by colours in both."""
+    rp, kc, colors = lattice(65, 65, 13, BOX, 2)
+    n = rp.size - 1
+    h = pmg.Handle(1, pmg.default_params(precision=first))
+    h.set_level_csr(0, rp, kc, n)
+    h.set_row_colors(0, colors, 8)
+    h.set_matrix(0, np.where(np.repeat(np.arange(n), np.diff(rp)) == kc, 60.0, -1.0))
+    assert step_launches(pmg, h, 0, first) == (6 if first else 15)
+    assert step_launches(pmg, h, 0, 1 - first) == 15
+    h.close()
