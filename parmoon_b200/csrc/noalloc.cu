@@ -72,8 +72,9 @@ __global__ void __launch_bounds__(256) k_defect_partials(int N, int R, const int
     const int row = row0 + rr;
     double s = 0.0, fr = 0.0;
     if (row < N) {
-      const int end = __ldg(rp + row + 1);
-      int k = __ldg(rp + row) + lane;
+      // (unsigned: k and the steps ahead of it may pass 2^31 in the last rows)
+      const unsigned end = __ldg(rp + row + 1);
+      unsigned k = __ldg(rp + row) + lane;
       if (lane == 0) fr = __ldg(f + row);
       // the entries of U steps first, then their x: two round trips for U steps
       for (; k + (U - 1) * W < end; k += U * W) {
