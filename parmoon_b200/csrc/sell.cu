@@ -1500,12 +1500,13 @@ static int sweep_colours(cudaStream_t s, const Level &L, bool forward, int mode,
 // always 0.)  Where two rows of one colour are coupled (sell_coupled) a repeated
 // update does change x, and none is left out.
 //
-// By blocks, one phase is a product over the whole GPU for what comes from
-// outside and one launch for the phase's own colours: 27 colours in 3 phases are 8
-// launches per step instead of 53.  Measured (64^3 Q2 hierarchy, FP32 / FP64
-// V-cycle): one launch per colour over whole rows 3.60 / 4.71 ms, over the split
-// rows 3.4 / 4.5, by blocks 2.25 / 3.5.  On the finest level (2.1 M rows) a phase
-// takes 31-51 us for the outside part (100 / 200 MB; 3.5-3.9 TB/s, bound by the
+// By blocks (where block_gain says so), one phase is a product over the whole GPU
+// for what comes from outside and one launch for the phase's own colours: 27 colours
+// in 3 phases are 10 launches for a step on an arbitrary x, 9 from x = 0 and 8 after
+// another step, instead of 53 (52 after another step).  Measured (64^3 Q2 hierarchy,
+// FP32 / FP64 V-cycle): one launch per colour over whole rows 3.60 / 4.71 ms, over the
+// split rows 3.4 / 4.5, by blocks 2.25 / 3.56, by blocks but for the finest FP64 level
+// 3.09.  On the finest level (2.1 M rows) a phase takes 31-51 us for the outside part (100 / 200 MB; 3.5-3.9 TB/s, bound by the
 // latency of short rows) and 24 us for its 9 colours (43 planes on 43 SMs); on
 // the 36 k-row level 3.5 + 4.3 us, where 9 colour launches took 23 us.
 template <typename T>

@@ -3,8 +3,8 @@
 //   vcycle          TMultiGrid3D::Cycle (src/FE/MultiGrid3D.C:449-695) with
 //                   step-length control off; FP64 or FP32 storage/compute
 //   coarse solve    SolveExact (src/FE/MGLevel3D.C:865-906): the explicit inverse
-//                   of the coarsest matrix (Gauss-Jordan with partial pivoting),
-//                   so each V-cycle applies one dense GEMV
+//                   of the coarsest matrix (Gauss-Jordan with partial pivoting and
+//                   one Newton step), so each V-cycle applies one dense GEMV
 //   preconditioner  TMultiGridScaIte::Iterate (src/FE/MultiGridScaIte.C:89-130)
 //   fgmres          TFgmresIte::Iterate, flexible branch (src/FE/FgmresIte.C:245-624):
 //                   right preconditioning, modified Gram-Schmidt, Givens rotations.
@@ -157,7 +157,7 @@ __global__ void k_gj_finish(int n, const double *__restrict__ M, const int *__re
 }
 
 // One Newton step X + X (I - A X) after the exchange steps: these alone leave 1.3
-// to 1.6 times the error of an LU with substitution, the step brings it below
+// to 3 times the error of an LU with substitution, the step brings it below
 // that (what is left is the rounding of X).  A X from the sparse rows, in twice the
 // working precision (exact products by FMA, sums with their rounding errors kept),
 // because the residual is all rounding; X R in FP64.  norm: the largest row sum of
@@ -933,8 +933,9 @@ int solve(Handle &h, double *sol_host, const double *rhs_host, pmg_solve_stats *
       // w = A z_i.  The solve copy holds no Dirichlet columns, and none are
       // needed: the start vector carries the Dirichlet values (copied above),
       // so the residual and every Krylov vector are exactly 0 on the
-      // Dirichlet rows (identity rows), and every smoother copies f_D = 0
-      // into x_D, so z_i is exactly 0 there too and A_aD z_D adds nothing
+      // Dirichlet rows (identity rows).  k_prec_in* sets x_D = f_D = 0 there and
+      // neither smoothers nor the prolongation touch these rows, so z_i is
+      // exactly 0 there too and A_aD z_D adds nothing
       PMG_TRY(sell_spmv<double>(s, F, zi, nullptr, w, 0, h.num_sms));
       double *Hc = Hd + (size_t)i * (m + 1);
       // modified Gram-Schmidt (FgmresIte.C): h_k = w.v_k, w -= h_k v_k for
@@ -1280,8 +1281,8 @@ extern "C" int pmg_vcycle(pmg_handle hh, const double *v_dev, double *z_dev) {
   PMG_TRY(pmg::prepare_levels(*h));
   PMG_TRY(pmg::capture_vcycle(*h));
   // the cycle takes f_D = 0: fold the Dirichlet part of v into the active
-  // rows in FP64 (f_a = v_a - A_aD v_D, f_D = 0), the cycle then keeps
-  // z_D = v_D as the smoothers' x_D = f_D did
+  // rows in FP64 (f_a = v_a - A_aD v_D, f_D = 0), the cycle then keeps x_D = 0
+  // and z_D = v_D is set behind it
   pmg::Level &F = h->lv.back();
   PMG_TRY(h->w.alloc(std::max<size_t>(h->w.n, (size_t)F.N)));
   double *f = h->w.p;

@@ -375,7 +375,7 @@ int mgs_step(Handle &h, size_t n, const double *hk_dev, const double *vk, const 
 // an exchange of sums between all SMs takes 4.4 us, a launch 3.)
 // The partial sums are added in a fixed order by every block for itself.
 constexpr int GS_THREADS = 512;
-constexpr int GS_K = 8;  // vectors per pass over w: 16 sums in registers, 9 loads in flight
+constexpr int GS_K = 8;  // vectors per pass over w: 16 sums in registers, 10 loads in flight (8 vectors, w, v_i)
 constexpr int GS_MAX = 61;
 
 __device__ inline double gs_partials(const double *part, int nblk, int lane) {
