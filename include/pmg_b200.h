@@ -86,7 +86,7 @@ typedef struct pmg_coeff_desc {
 #define PMG_COARSE_JACOBI     1
 #define PMG_COARSE_SOR        2
 #define PMG_COARSE_SSOR       3
-#define PMG_COARSE_DIRECT    17  /* dense LU of the coarsest level (reference: SolveExact) */
+#define PMG_COARSE_DIRECT    17  /* dense inverse of the coarsest level (reference: SolveExact) */
 #define PMG_PREC_FP64         0  /* V-cycle stores level matrices and vectors in FP64 */
 #define PMG_PREC_FP32         1  /* V-cycle in FP32, outer FGMRES / true residual in FP64 */
 
@@ -434,7 +434,7 @@ int pmg_last_timings(pmg_handle h, double *assemble_s, double *solve_s, double *
 #define PMG_KERNEL_SSOR32    3
 #define PMG_KERNEL_ASSEMBLE  4
 #define PMG_KERNEL_CSR_SPMV64 5
-#define PMG_KERNEL_COARSE_FACTOR 6  /* LU + inverse of the coarsest level (level must be 0) */
+#define PMG_KERNEL_COARSE_FACTOR 6  /* dense inverse of the coarsest level (level must be 0) */
 #define PMG_KERNEL_LEARNED_FWD 7    /* the stencil network's forward on the level's lattice (features, three
                                        tensor-core convolutions, stencil); flops = 2 x 27 x (27*32 + 32*32 +
                                        32*27) per lattice node; needs weights and a lattice */
